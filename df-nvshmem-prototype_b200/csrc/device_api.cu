@@ -25,11 +25,7 @@ __device__ __noinline__ void put_thread(T *target, const T *source, int len, int
   if (!nvshm::check_remote(c, target, bytes, pe) || !nvshm::check_local(c, source, bytes)) return;
   char *dst = nvshm::xlate(c, target, pe);
   unsigned long long t0 = c.trace ? nvshm::gtimer() : 0;
-  // one thread: 16 vector accesses in flight (measured 2.6x the bandwidth of 4
-  // for a 1 MiB put, 2.2x on a batch of calls, at 90 instead of 54 registers),
-  // and an L2 prefetch 64 rounds (16 KiB) ahead: 1 MiB from DRAM 0.90 -> 1.36
-  // GB/s, from L2 1.89 -> 1.81 GB/s; the C4 batch of calls 351 -> 486 GB/s
-  nvshm::copy_coop<16, 16, 64>(dst, reinterpret_cast<const char *>(source), bytes, 0, 1);
+  nvshm::copy_lanes<8, 8>(dst, reinterpret_cast<const char *>(source), bytes);
   if (c.trace) nvshm::trace_rec(c, op, source, dst, bytes, pe, t0, nvshm::gtimer());
 }
 
@@ -40,7 +36,7 @@ __device__ __noinline__ void get_thread(T *target, const T *source, int len, int
   if (!nvshm::check_remote(c, source, bytes, pe) || !nvshm::check_local(c, target, bytes)) return;
   const char *src = nvshm::xlate(c, source, pe);
   unsigned long long t0 = c.trace ? nvshm::gtimer() : 0;
-  nvshm::copy_coop<16, 16, 64>(reinterpret_cast<char *>(target), src, bytes, 0, 1);
+  nvshm::copy_lanes<8, 8>(reinterpret_cast<char *>(target), src, bytes);
   if (c.trace) nvshm::trace_rec(c, op, target, src, bytes, pe, t0, nvshm::gtimer());
 }
 

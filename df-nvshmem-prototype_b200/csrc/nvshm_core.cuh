@@ -91,6 +91,12 @@ __device__ __forceinline__ unsigned smem_u32(const void *p) {
   return (unsigned)__cvta_generic_to_shared(p);
 }
 
+__device__ __forceinline__ unsigned lane_number() {
+  unsigned l;
+  asm("mov.u32 %0, %%laneid;" : "=r"(l));
+  return l;
+}
+
 // ------------------------------------------------------------- PE / addresses
 // The calling PE: blockIdx.z of a collective launch, or the process's PE when
 // every PE is a process of its own.
@@ -170,16 +176,87 @@ __device__ __forceinline__ void l2_prefetch_bulk(uintptr_t p, unsigned bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes));
 }
 
+// 16 bytes whose address is only LB-byte aligned.  LB 4 stands for addresses
+// that are 4 modulo 8 (one that is 0 modulo 8 takes LB 8), so the middle two
+// words are one 8-byte load; LB 1 for addresses that are not 0 modulo 4.
+template <int LB>
+__device__ __forceinline__ uint4 load16(const char *p) {
+  if (LB == 16) return *reinterpret_cast<const uint4 *>(p);
+  uint4 v;
+  if (LB == 1) {
+    // the five words that hold the 16 bytes, shifted; each of them holds at
+    // least one of the bytes, so none lies outside the source's words
+    const unsigned *q = reinterpret_cast<const unsigned *>((uintptr_t)p & ~(uintptr_t)3);
+    const unsigned sh = ((unsigned)(uintptr_t)p & 3u) * 8u;
+    const unsigned w0 = q[0], w1 = q[1], w2 = q[2], w3 = q[3], w4 = q[4];
+    v.x = __funnelshift_r(w0, w1, sh), v.y = __funnelshift_r(w1, w2, sh);
+    v.z = __funnelshift_r(w2, w3, sh), v.w = __funnelshift_r(w3, w4, sh);
+  } else if (LB == 8) {
+    const uint2 a = *reinterpret_cast<const uint2 *>(p), b = *reinterpret_cast<const uint2 *>(p + 8);
+    v.x = a.x, v.y = a.y, v.z = b.x, v.w = b.y;
+  } else {
+    v.x = *reinterpret_cast<const unsigned *>(p);
+    const uint2 m = *reinterpret_cast<const uint2 *>(p + 4);
+    v.y = m.x, v.z = m.y;
+    v.w = *reinterpret_cast<const unsigned *>(p + 12);
+  }
+  return v;
+}
+
+// The first `have` of U vectors 512 bytes apart; the loads' width follows the
+// relative alignment `mis` (the same for the whole warp), in one set of
+// registers for the three widths.
+template <int U>
+__device__ __forceinline__ void load_row(uint4 *v, const char *s, unsigned mis, unsigned have) {
+  if ((mis & 15) == 0) {
+#pragma unroll
+    for (unsigned u = 0; u < U; ++u)
+      if (u < have) v[u] = load16<16>(s + u * 512);
+  } else if ((mis & 7) == 0) {
+#pragma unroll
+    for (unsigned u = 0; u < U; ++u)
+      if (u < have) v[u] = load16<8>(s + u * 512);
+  } else if ((mis & 3) == 0) {
+#pragma unroll
+    for (unsigned u = 0; u < U; ++u)
+      if (u < have) v[u] = load16<4>(s + u * 512);
+  } else if (U <= 4) {
+#pragma unroll
+    for (unsigned u = 0; u < U; ++u)
+      if (u < have) v[u] = load16<1>(s + u * 512);
+  }
+}
+
+// One VB-byte vector of a source that is LB-byte aligned (LB < VB: VB is 16).
+template <int VB, int LB>
+__device__ __forceinline__ typename VecT<VB>::T load_vec(const typename VecT<VB>::T *p) {
+  return *p;
+}
+template <>
+__device__ __forceinline__ uint4 load_vec<16, 8>(const uint4 *p) {
+  return load16<8>(reinterpret_cast<const char *>(p));
+}
+template <>
+__device__ __forceinline__ uint4 load_vec<16, 4>(const uint4 *p) {
+  return load16<4>(reinterpret_cast<const char *>(p));
+}
+
 // Copies `bytes` with `nthr` cooperating threads (this one is `r`), VB-byte
-// accesses for the aligned body and U accesses in flight per thread.  dst and
-// src must have the same alignment modulo VB.
+// stores for the body aligned to the destination and U accesses in flight per
+// thread.  LB is the alignment of the source there: with LB < VB a vector is
+// put together from two or three narrower loads, so a copy between arrays
+// that lie 4, 8 or 12 bytes apart modulo 16 still stores whole vectors and
+// keeps 16 bytes in flight per access (before, it went by 4- or 8-byte
+// accesses both ways: 1500 one-CTA puts of 140 KB at 4-byte offsets took
+// 148 us, now 95 us; the narrower loads of one vector share L1 sectors, so
+// L2 and DRAM see each byte once).
 //
 // PFI > 0: a copy by one thread or one warp is bound by the latency of its
 // loads (U accesses per thread per round).  Its thread 0 keeps an L2
 // prefetch of the source PFI rounds in front of the loads (never past the
 // source range), so the loads hit L2 instead of DRAM.  Copies shorter than
 // twice that distance skip it.
-template <int VB, int U, unsigned PFI = 0>
+template <int VB, int U, unsigned PFI = 0, int LB = VB>
 __device__ __forceinline__ void copy_body(char *__restrict__ dst, const char *__restrict__ src,
                                           unsigned long long bytes, unsigned r, unsigned nthr) {
   typedef typename VecT<VB>::T V;
@@ -196,10 +273,11 @@ __device__ __forceinline__ void copy_body(char *__restrict__ dst, const char *__
   const uintptr_t pf_end = ((uintptr_t)src + bytes) & ~(uintptr_t)15;
   uintptr_t pf = ((uintptr_t)src + 15) & ~(uintptr_t)15;  // next source byte to stage
   if (nv >= (unsigned long long)(U - 1) * nthr) {
+#pragma unroll 1
     for (; i + (unsigned long long)(U - 1) * nthr < nv; i += step) {
       V v[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) v[u] = s[i + (unsigned long long)u * nthr];
+      for (int u = 0; u < U; ++u) v[u] = load_vec<VB, LB>(s + i + (unsigned long long)u * nthr);
       // between this iteration's loads and its stores: the stores of one
       // iteration and the loads of the next stay free to interleave
       // (measured: placed before the loads, the prefetch cost 15-23% on
@@ -219,31 +297,314 @@ __device__ __forceinline__ void copy_body(char *__restrict__ dst, const char *__
   }
   // copies too short for U accesses per thread still get 4 in flight
   if (U > 4) {
+#pragma unroll 1
     for (; i + 3ull * nthr < nv; i += 4ull * nthr) {
       V v[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = s[i + (unsigned long long)u * nthr];
+      for (int u = 0; u < 4; ++u) v[u] = load_vec<VB, LB>(s + i + (unsigned long long)u * nthr);
 #pragma unroll
       for (int u = 0; u < 4; ++u) d[i + (unsigned long long)u * nthr] = v[u];
     }
   }
-  for (; i < nv; i += nthr) d[i] = s[i];
+#pragma unroll 1
+  for (; i < nv; i += nthr) d[i] = load_vec<VB, LB>(s + i);
   for (unsigned long long j = head + nv * VB + r; j < bytes; j += nthr) dst[j] = src[j];
 }
 
-// Widest access the relative alignment of dst and src allows, capped at MAXV.
+// The body of a copy by whole warps (n >= 32 threads, of which the full warps
+// take part): nv 16-byte vectors from an LB-byte aligned source, in tiles of
+// U x 32 consecutive vectors, a warp per tile.  Within a tile every access is
+// at a constant distance from the first, so a lane holds two addresses and U
+// vectors (a stride known only at run time costs an address pair for each of
+// the U accesses both ways: 72 instead of 60 registers for U = 8).
+// PFI > 0: a lone warp keeps an L2 prefetch PFI tiles ahead (see copy_body).
+template <int U, unsigned PFI>
+__device__ __forceinline__ void copy_tiles(char *__restrict__ dst, const char *__restrict__ src,
+                                           unsigned long long nv, unsigned mis, unsigned r, unsigned n) {
+  constexpr unsigned TB = U * 512;  // bytes per tile
+  const unsigned nw = n >> 5, w = r >> 5, lane = r & 31u;
+  // operands a number of bytes apart: in rows of four only (load_row)
+  const unsigned long long ntiles = (mis & 3) == 0 ? nv / (U * 32) : 0;
+  const bool pf_on = PFI > 0 && n == 32 && lane == 0 && ntiles >= 2ull * PFI;
+  const uintptr_t pf_end = ((uintptr_t)src + nv * 16) & ~(uintptr_t)15;
+  uintptr_t pf = ((uintptr_t)src + 15) & ~(uintptr_t)15;  // next source byte to stage
+  const char *s = src + (unsigned long long)w * TB + lane * 16u;
+  char *d = dst + (unsigned long long)w * TB + lane * 16u;
+  if (w < nw) {
+#pragma unroll 1
+    for (unsigned long long t = w; t < ntiles; t += nw) {
+      uint4 v[U];
+      load_row<U>(v, s, mis, U);
+      if (pf_on) {
+        uintptr_t want = ((uintptr_t)s + PFI * TB) & ~(uintptr_t)15;
+        if (want > pf_end) want = pf_end;
+        if (want >= pf + 4096 || (want == pf_end && want > pf)) {
+          const unsigned k = (unsigned)(want - pf < 65536 ? want - pf : 65536);
+          l2_prefetch_bulk(pf, k);
+          pf += k;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) *reinterpret_cast<uint4 *>(d + u * 512) = v[u];
+      s += (unsigned long long)nw * TB;
+      d += (unsigned long long)nw * TB;
+    }
+  }
+  // the vectors after the last whole tile: rounds of 4 rows of 32 for a warp,
+  // the same rows dealt out over the warps of a block
+  const unsigned long long left = nv - ntiles * (U * 32);
+  s = src + ntiles * TB + 16u * lane;
+  d = dst + ntiles * TB + 16u * lane;
+  if (w < nw) {
+#pragma unroll 1
+    for (unsigned long long i = w * 128; i < left; i += nw * 128) {
+      uint4 v[4];
+      const unsigned rows = left - i < 128 ? (unsigned)(left - i) : 128u;  // vectors of this round
+      const unsigned have = rows > lane ? (rows - lane + 31) / 32 : 0;     // this lane's
+      load_row<4>(v, s + i * 16, mis, have);
+#pragma unroll
+      for (unsigned u = 0; u < 4; ++u)
+        if (u < have) *reinterpret_cast<uint4 *>(d + i * 16 + u * 512) = v[u];
+    }
+  }
+}
+
+// One thread, one warp or a block copies `bytes`: 16-byte stores, with loads
+// as wide as the relative alignment of dst and src allows.  MAXV caps the
+// width of both (4 and 8: the batch engine's narrow configurations).
 template <int MAXV = 16, int U = 4, unsigned PFI = 0>
 __device__ __forceinline__ void copy_coop(char *dst, const char *src, unsigned long long bytes,
                                           unsigned r, unsigned nthr) {
   const unsigned mis = (unsigned)((uintptr_t)dst ^ (uintptr_t)src);
-  if (MAXV >= 16 && (mis & 15) == 0)
-    copy_body<16, U, PFI>(dst, src, bytes, r, nthr);
-  else if (MAXV >= 8 && (mis & 7) == 0)
-    copy_body<8, U, PFI>(dst, src, bytes, r, nthr);
-  else if ((mis & 3) == 0)
-    copy_body<4, U, PFI>(dst, src, bytes, r, nthr);
-  else
-    copy_body<1, U, PFI>(dst, src, bytes, r, nthr);
+  if (MAXV < 16) {
+    if (MAXV == 8 && (mis & 7) == 0)
+      copy_body<8, U, PFI>(dst, src, bytes, r, nthr);
+    else if ((mis & 3) == 0)
+      copy_body<4, U, PFI>(dst, src, bytes, r, nthr);
+    else
+      copy_body<1, U, PFI>(dst, src, bytes, r, nthr);
+    return;
+  }
+  if (nthr < 32) {
+    if ((mis & 3) != 0)
+      copy_body<1, 4>(dst, src, bytes, r, nthr);
+    else if ((mis & 15) == 0)
+      copy_body<16, U, PFI>(dst, src, bytes, r, nthr);
+    else if ((mis & 7) == 0)
+      copy_body<16, U, PFI, 8>(dst, src, bytes, r, nthr);
+    else
+      copy_body<16, U, PFI, 4>(dst, src, bytes, r, nthr);
+    return;
+  }
+  unsigned head = (unsigned)(16 - ((uintptr_t)dst & 15)) & 15u;
+  if (head > bytes) head = (unsigned)bytes;
+  const unsigned long long nv = (bytes - head) >> 4;
+  const unsigned tail = (unsigned)(bytes - head) & 15u;
+  // fewer than 32 edge bytes: one each
+  if (r < head) dst[r] = src[r];
+  if (r >= 16 && r - 16 < tail) {
+    const unsigned long long j = bytes - tail + (r - 16);
+    dst[j] = src[j];
+  }
+  dst += head;
+  src += head;
+  copy_tiles<U, PFI>(dst, src, nv, mis, r, nthr);
+}
+
+// ----------------------------------------------- one copy per thread, shared
+// A long copy by a whole warp: U vectors in flight per lane and the source
+// prefetched into L2 `kAhead` bytes in front of the loads, which a lone warp
+// waits for in every round.  Copies the whole rounds of U * 32 vectors and
+// returns how many vectors that was.  (Two or three sets of 8 vectors in
+// rotation, so that loads stay in flight while a set is stored, measured no
+// better: they need the registers of U = 16 or 24 at once.)
+constexpr unsigned kAhead = 32768;
+
+template <int U>
+__device__ __forceinline__ unsigned copy_warp_long(unsigned lane, char *dst, const char *src, unsigned nv,
+                                                   unsigned mis) {
+  const unsigned rounds = nv / (U * 32);
+  const uintptr_t pf_end = ((uintptr_t)src + (unsigned long long)nv * 16u) & ~(uintptr_t)15;
+  uintptr_t pf = ((uintptr_t)src + 15) & ~(uintptr_t)15;
+  const char *s = src + 16u * lane;
+  char *d = dst + 16u * lane;
+#pragma unroll 1
+  for (unsigned k = 0; k < rounds; ++k) {
+    uint4 v[U];
+    load_row<U>(v, s, mis, U);
+    if (lane == 0) {
+      uintptr_t want = ((uintptr_t)s + kAhead) & ~(uintptr_t)15;
+      if (want > pf_end) want = pf_end;
+      if (want >= pf + 4096) {
+        l2_prefetch_bulk(pf, (unsigned)(want - pf));
+        pf = want;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) *reinterpret_cast<uint4 *>(d + u * 512) = v[u];
+    s += U * 512;
+    d += U * 512;
+  }
+  return rounds * U * 32;
+}
+
+// The calling lanes' copies of one load alignment as one stream of 16-byte
+// vectors: the lanes of `mask` (this one is number `r` of `nl`) take the
+// messages of `todo` one after the other, nl vectors of one message per slot
+// and U slots in flight, so U short messages or U * nl vectors of a long one
+// are read at once.  dst / src / nv are this lane's own message.  One pass per
+// alignment: with the width chosen per slot instead, the branches between the
+// loads keep them from overlapping (25,000 calls: 215 us against 115-140 us).
+template <int LB, int U>
+__device__ __forceinline__ void copy_lanes_body(unsigned mask, unsigned todo, unsigned r, unsigned nl, char *dst,
+                                                const char *src, unsigned nv) {
+  unsigned long long cd = 0, cs = 0;  // the current message, at this lane's vector
+  unsigned left = 0;                  // its vectors from lane 0's on
+#pragma unroll 1
+  while (left > 0 || todo) {
+    uint4 v[U];
+    uint4 *d[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      d[u] = nullptr;
+      if (left == 0 && todo) {
+        const int o = __ffs(todo) - 1;
+        todo &= todo - 1;
+        cd = __shfl_sync(mask, (unsigned long long)dst, o) + 16ull * r;
+        cs = __shfl_sync(mask, (unsigned long long)src, o) + 16ull * r;
+        left = __shfl_sync(mask, nv, o);
+      }
+      if (r < left) {
+        d[u] = reinterpret_cast<uint4 *>(cd);
+        v[u] = load16<LB>(reinterpret_cast<const char *>(cs));
+      }
+      cd += 16ull * nl;
+      cs += 16ull * nl;
+      left = left > nl ? left - nl : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (d[u]) *d[u] = v[u];
+  }
+}
+
+// kOwn: a lane copies up to this many vectors itself (one round trip, in
+// parallel with the other lanes); kLong: from this many on (16 KiB) a copy is
+// a long one; kTogether: fewer lanes than this copy alone (together they
+// would have less in flight than each with 16 accesses of its own).
+constexpr unsigned kOwn = 4, kLong = 1024, kTogether = 16;
+
+// One copy by a warp, its long part with U vectors in flight per lane.
+template <int U>
+__device__ __forceinline__ void copy_warp(char *dst, const char *src, unsigned long long bytes, unsigned lane) {
+  const unsigned mis = (unsigned)((uintptr_t)dst ^ (uintptr_t)src);
+  if (bytes >= kLong * 16 && (mis & 3) == 0) {
+    const unsigned head = (unsigned)(16 - ((uintptr_t)dst & 15)) & 15u;
+    if (lane < head) dst[lane] = src[lane];
+    const unsigned nv = (unsigned)((bytes - head) >> 4);
+    const unsigned long long done = head + 16ull * copy_warp_long<U>(lane, dst + head, src + head, nv, mis);
+    dst += done;
+    src += done;
+    bytes -= done;
+  }
+  copy_coop<16, 8>(dst, src, bytes, lane, 32);
+}
+
+template <int LB>
+__device__ __forceinline__ void copy_own(char *dst, const char *src, unsigned nv) {
+  uint4 v[kOwn];
+#pragma unroll
+  for (unsigned k = 0; k < kOwn; ++k)
+    if (k < nv) v[k] = load16<LB>(src + 16 * k);
+#pragma unroll
+  for (unsigned k = 0; k < kOwn; ++k)
+    if (k < nv) reinterpret_cast<uint4 *>(dst)[k] = v[k];
+}
+
+// One copy per calling thread (the thread forms of put and get).  Lanes of a
+// warp that arrive together carry their copies out together: a lane alone
+// keeps at most 16 accesses in flight and touches a line of its own each
+// time, while the group reads whole lines and has its accesses wherever there
+// is work (see copy_lanes_body).  25,000 calls of log-normal sizes (median
+// 2 KiB, up to 3 MiB, 282 MB moved) took 1240-2060 us with every lane on its
+// own, as long as the longest call takes one thread; together 115-140 us.
+// A lane whose copy has at most kOwn vectors, or operands that are not 4-byte
+// aligned, copies it itself, as do fewer than kTogether lanes.  LU / SU: the
+// vectors in flight per lane for long and short copies.  FULL: the caller
+// knows that all 32 lanes are here.
+//
+// The first __syncwarp makes what a lane wrote before its call visible to the
+// lanes that copy for it, the last one makes their stores the calling lane's
+// (its later fences and signals order them like its own).
+template <int LU, int SU, bool FULL = false>
+__device__ __forceinline__ void copy_lanes(char *dst, const char *src, unsigned long long bytes) {
+  const unsigned mask = FULL ? 0xffffffffu : __activemask();
+  const unsigned nl = FULL ? 32u : __popc(mask);
+  const unsigned mis = (unsigned)((uintptr_t)dst ^ (uintptr_t)src);
+  if (!FULL && nl < kTogether) {
+    // one thread: 16 vector accesses in flight (measured 2.6x the bandwidth of
+    // 4 for a 1 MiB put) and an L2 prefetch 64 rounds (16 KiB) ahead: 1 MiB
+    // from DRAM 0.90 -> 1.36 GB/s, from L2 1.89 -> 1.81 GB/s
+    copy_coop<16, 16, 64>(dst, src, bytes, 0, 1);
+    return;
+  }
+  __syncwarp(mask);
+  unsigned nv = 0;
+  if (((mis | (unsigned)(uintptr_t)dst | (unsigned)bytes) & 3) != 0) {
+    copy_coop<16, 4>(dst, src, bytes, 0, 1);
+  } else {
+    // the words before and after the 16-byte vectors of the destination
+    unsigned head = (unsigned)(16 - ((uintptr_t)dst & 15)) & 15u;
+    if (head > bytes) head = (unsigned)bytes;
+    nv = (unsigned)((bytes - head) >> 4);
+    const unsigned tail = (unsigned)(bytes - head) & 15u;
+    const char *ts = src + (bytes - tail);
+    char *td = dst + (bytes - tail);
+    unsigned w[6];
+#pragma unroll
+    for (unsigned k = 0; k < 3; ++k) {
+      if (4 * k < head) w[k] = reinterpret_cast<const unsigned *>(src)[k];
+      if (4 * k < tail) w[3 + k] = reinterpret_cast<const unsigned *>(ts)[k];
+    }
+#pragma unroll
+    for (unsigned k = 0; k < 3; ++k) {
+      if (4 * k < head) reinterpret_cast<unsigned *>(dst)[k] = w[k];
+      if (4 * k < tail) reinterpret_cast<unsigned *>(td)[k] = w[3 + k];
+    }
+    dst += head;
+    src += head;
+    if (nv <= kOwn) {
+      if ((mis & 15) == 0)
+        copy_own<16>(dst, src, nv);
+      else if ((mis & 7) == 0)
+        copy_own<8>(dst, src, nv);
+      else
+        copy_own<4>(dst, src, nv);
+      nv = 0;
+    }
+  }
+  const unsigned r = __popc(mask & ((1u << lane_number()) - 1u));
+  if (mask == 0xffffffffu) {
+#pragma unroll 1
+    for (unsigned todo = __ballot_sync(mask, nv >= kLong); todo; todo &= todo - 1) {
+      const int o = __ffs(todo) - 1;
+      char *d = (char *)__shfl_sync(mask, (unsigned long long)dst, o);
+      const char *p = (const char *)__shfl_sync(mask, (unsigned long long)src, o);
+      const unsigned k = copy_warp_long<LU>(r, d, p, __shfl_sync(mask, nv, o), __shfl_sync(mask, mis, o));
+      if ((int)r == o) {
+        nv -= k;
+        dst += 16ull * k;
+        src += 16ull * k;
+      }
+    }
+  }
+  const unsigned lb = (mis & 15) == 0 ? 16 : ((mis & 7) == 0 ? 8 : 4);
+  const unsigned t16 = __ballot_sync(mask, nv && lb == 16), t8 = __ballot_sync(mask, nv && lb == 8),
+                 t4 = __ballot_sync(mask, nv && lb == 4);
+  copy_lanes_body<16, SU>(mask, t16, r, nl, dst, src, nv);
+  copy_lanes_body<8, SU>(mask, t8, r, nl, dst, src, nv);
+  copy_lanes_body<4, SU>(mask, t4, r, nl, dst, src, nv);
+  __syncwarp(mask);
 }
 
 __device__ __forceinline__ unsigned block_rank() {

@@ -60,11 +60,60 @@ __device__ __forceinline__ char *slice_ptr(const Cfg &c, int pe, unsigned long l
 
 // ------------------------------------------------------------ request lists
 // One caller unit per request: a thread (MODE_THREAD), a warp (MODE_WARP) or
-// a CTA (MODE_BLOCK / MODE_BULK).  The symmetric operand is passed as PE 0's
+// a CTA (MODE_BLOCK / MODE_BULK).  The symmetric operand is named by PE 0's
 // copy of the object (any slice names the same object).
+
+// A PUT or GET: the checks, translation, copy and trace record of the public
+// put and get, written once for all operations and types.  In the thread form
+// the lanes of a warp so reach the shared copy together (branching to the six
+// typed calls would split them into groups); in the other forms the copy is
+// part of the kernel, which has registers for more accesses in flight.
 template <int MODE>
-__global__ void exec_requests_kernel(Cfg c, const nvshmemx_request *__restrict__ reqs, int n,
-                                     unsigned bulk_smem) {
+__device__ __forceinline__ void copy_request(const Cfg &c, const nvshmemx_request &r, char *smem, unsigned bulk_smem) {
+  const bool put = r.op == NVSHMEMX_REQ_PUT;
+  unsigned long long bytes = r.dtype == NVSHMEMX_DT_DOUBLE   ? r.bytes & ~7u
+                             : r.dtype < NVSHMEMX_DT_DOUBLE ? r.bytes & ~3u
+                                                            : (r.bytes >> 2) * 8ull;
+  char *near = slice_ptr(c, put ? r.src_pe : r.dst_pe, put ? r.src_off : r.dst_off);
+  const char *sym = c.arena + (put ? r.dst_off : r.src_off);
+  const int pe = put ? r.dst_pe : r.src_pe;
+  bool ok = r.op <= NVSHMEMX_REQ_GET;
+  ok = ok && check_remote(c, sym, bytes, pe) && check_local(c, near, bytes);
+  if (MODE == NVSHMEMX_MODE_THREAD) {
+    if (!ok) bytes = 0;
+  } else if (!ok) {
+    return;
+  }
+  char *far = xlate(c, sym, pe);
+  char *dst = put ? far : near;
+  const char *src = put ? near : far;
+  const bool rec = ok && c.trace && MODE != NVSHMEMX_MODE_BULK &&
+                   (MODE == NVSHMEMX_MODE_THREAD ||
+                    (MODE == NVSHMEMX_MODE_WARP ? (threadIdx.x & 31) == 0 : threadIdx.x == 0));
+  const unsigned long long t0 = rec ? gtimer() : 0;
+  if (MODE == NVSHMEMX_MODE_THREAD)
+    copy_lanes<16, 8, true>(dst, src, bytes);
+  else if (MODE == NVSHMEMX_MODE_WARP)
+    copy_warp<12>(dst, src, bytes, threadIdx.x & 31);
+  else if (MODE == NVSHMEMX_MODE_BLOCK)
+    copy_coop<16, 8>(dst, src, bytes, threadIdx.x, blockDim.x);
+  else
+    bulk_copy_block(c, dst, src, bytes, smem, bulk_smem);
+  if (rec) {
+    const int op = (put ? NVSHMEMX_TRACE_PUT_INT : NVSHMEMX_TRACE_GET_INT) + (r.dtype < 2 ? (int)r.dtype : 2);
+    trace_rec(c, op, near, far, bytes, pe, t0, gtimer());
+  }
+}
+
+// CTAs of two warps in the thread and warp forms: a CTA's place frees up with
+// its longest request, and 25,000 one-thread requests still give every SM
+// work.  The warp form runs 20 warps per SM with 12 vectors in flight each:
+// 100,000 requests 255-270 us, against 300-360 us with 24 warps of 8 vectors
+// in CTAs of eight (its largest request, one warp's, is a third of that time).
+template <int MODE>
+__global__ void __launch_bounds__(MODE <= NVSHMEMX_MODE_WARP ? 64 : 256,
+                                  MODE == NVSHMEMX_MODE_THREAD ? 8 : MODE == NVSHMEMX_MODE_WARP ? 10 : 3)
+    exec_requests_kernel(Cfg c, const nvshmemx_request *__restrict__ reqs, int n, unsigned bulk_smem) {
   extern __shared__ __align__(128) char smem[];
   long long u;
   if (MODE == NVSHMEMX_MODE_THREAD)
@@ -73,53 +122,29 @@ __global__ void exec_requests_kernel(Cfg c, const nvshmemx_request *__restrict__
     u = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   else
     u = blockIdx.x;
-  if (u >= n) return;
-  const nvshmemx_request r = reqs[u];
+  nvshmemx_request r;
+  if (MODE == NVSHMEMX_MODE_THREAD) {
+    // every lane takes part in the warp's copies, those without one too
+    r.op = 0xff;
+    r.bytes = 0;
+    r.dtype = 0;
+    r.src_pe = r.dst_pe = 0;
+    r.src_off = r.dst_off = 0;
+    if (u < n) r = reqs[u];
+    copy_request<MODE>(c, r, smem, bulk_smem);
+    if (u >= n || r.op <= NVSHMEMX_REQ_GET) return;
+  } else {
+    if (u >= n) return;
+    r = reqs[u];
+  }
   const bool leader = MODE == NVSHMEMX_MODE_THREAD || (MODE == NVSHMEMX_MODE_WARP ? (threadIdx.x & 31) == 0
                                                                                  : threadIdx.x == 0);
   const int w = r.dtype == NVSHMEMX_DT_DOUBLE ? 8 : 4;
-  const int len = (int)(r.bytes / (unsigned)w);
   switch (r.op) {
-    case NVSHMEMX_REQ_PUT: {
-      char *sym = c.arena + r.dst_off;
-      char *src = slice_ptr(c, r.src_pe, r.src_off);
-      if (MODE == NVSHMEMX_MODE_THREAD) {
-        if (r.dtype == NVSHMEMX_DT_INT) nvshmem_int_put((int *)sym, (int *)src, len, r.dst_pe);
-        else if (r.dtype == NVSHMEMX_DT_FLOAT) nvshmem_float_put((float *)sym, (float *)src, len, r.dst_pe);
-        else nvshmem_double_put((double *)sym, (double *)src, len, r.dst_pe);
-      } else if (MODE == NVSHMEMX_MODE_WARP) {
-        if (r.dtype == NVSHMEMX_DT_INT) nvshmemx_int_put_warp((int *)sym, (int *)src, len, r.dst_pe);
-        else if (r.dtype == NVSHMEMX_DT_FLOAT) nvshmemx_float_put_warp((float *)sym, (float *)src, len, r.dst_pe);
-        else nvshmemx_double_put_warp((double *)sym, (double *)src, len, r.dst_pe);
-      } else if (MODE == NVSHMEMX_MODE_BLOCK) {
-        if (r.dtype == NVSHMEMX_DT_INT) nvshmemx_int_put_block((int *)sym, (int *)src, len, r.dst_pe);
-        else if (r.dtype == NVSHMEMX_DT_FLOAT) nvshmemx_float_put_block((float *)sym, (float *)src, len, r.dst_pe);
-        else nvshmemx_double_put_block((double *)sym, (double *)src, len, r.dst_pe);
-      } else {
-        nvshmemx_putmem_bulk_block(sym, src, (size_t)len * w, r.dst_pe, smem, bulk_smem);
-      }
+    case NVSHMEMX_REQ_PUT:
+    case NVSHMEMX_REQ_GET:
+      copy_request<MODE>(c, r, smem, bulk_smem);
       break;
-    }
-    case NVSHMEMX_REQ_GET: {
-      char *sym = c.arena + r.src_off;
-      char *dst = slice_ptr(c, r.dst_pe, r.dst_off);
-      if (MODE == NVSHMEMX_MODE_THREAD) {
-        if (r.dtype == NVSHMEMX_DT_INT) nvshmem_int_get((int *)dst, (int *)sym, len, r.src_pe);
-        else if (r.dtype == NVSHMEMX_DT_FLOAT) nvshmem_float_get((float *)dst, (float *)sym, len, r.src_pe);
-        else nvshmem_double_get((double *)dst, (double *)sym, len, r.src_pe);
-      } else if (MODE == NVSHMEMX_MODE_WARP) {
-        if (r.dtype == NVSHMEMX_DT_INT) nvshmemx_int_get_warp((int *)dst, (int *)sym, len, r.src_pe);
-        else if (r.dtype == NVSHMEMX_DT_FLOAT) nvshmemx_float_get_warp((float *)dst, (float *)sym, len, r.src_pe);
-        else nvshmemx_double_get_warp((double *)dst, (double *)sym, len, r.src_pe);
-      } else if (MODE == NVSHMEMX_MODE_BLOCK) {
-        if (r.dtype == NVSHMEMX_DT_INT) nvshmemx_int_get_block((int *)dst, (int *)sym, len, r.src_pe);
-        else if (r.dtype == NVSHMEMX_DT_FLOAT) nvshmemx_float_get_block((float *)dst, (float *)sym, len, r.src_pe);
-        else nvshmemx_double_get_block((double *)dst, (double *)sym, len, r.src_pe);
-      } else {
-        nvshmemx_getmem_bulk_block(dst, sym, (size_t)len * w, r.src_pe, smem, bulk_smem);
-      }
-      break;
-    }
     case NVSHMEMX_REQ_SIGNAL:
       if (leader) nvshmemx_int_signal((int *)(c.arena + r.dst_off), r.value, r.dst_pe);
       break;
@@ -375,8 +400,11 @@ __device__ __forceinline__ bool a2a_stream_1t(const Cfg &c, char *smem, unsigned
 // contiguous, 16-byte-rounded segment per caller unit (warp or CTA), so every
 // unit streams one range; MODE_THREAD keeps the prototype's shape, one thread
 // per message through the typed per-thread call.
+// Bounds: as many threads and CTAs per SM as its callers may ask for (a thread
+// per message up to 289 PEs; two, with the ring's shared memory three, CTAs).
 template <int MODE>
-__global__ void alltoall_kernel(Cfg c, int op, int dtype, unsigned long long send_off,
+__global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 288 : 256, MODE == NVSHMEMX_MODE_BULK ? 3 : 2)
+    alltoall_kernel(Cfg c, int op, int dtype, unsigned long long send_off,
                                 unsigned long long recv_off, unsigned long long bytes, int rounds, int nsets,
                                 unsigned long long set_stride, unsigned bulk_smem, int device_barrier) {
   extern __shared__ __align__(128) char smem[];
@@ -393,28 +421,23 @@ __global__ void alltoall_kernel(Cfg c, int op, int dtype, unsigned long long sen
     unit = blockIdx.x;
     nunits = gridDim.x;
   }
-  const int w = dtype == NVSHMEMX_DT_DOUBLE ? 8 : 4;
   for (int r = 0; r < rounds; ++r) {
     const unsigned long long so = send_off + (unsigned long long)(r % nsets) * set_stride;
     const unsigned long long ro = recv_off + (unsigned long long)(r % nsets) * set_stride;
     if (MODE == NVSHMEMX_MODE_THREAD) {
-      if (unit < nunits) {
-        const int q = (pe + 1 + (int)unit) % np;
-        const int len = (int)(bytes / w);
-        if (op == NVSHMEMX_REQ_PUT) {
-          char *sym = c.arena + ro + (unsigned long long)pe * bytes;
-          char *src = slice_ptr(c, pe, so + (unsigned long long)q * bytes);
-          if (dtype == NVSHMEMX_DT_INT) nvshmem_int_put((int *)sym, (int *)src, len, q);
-          else if (dtype == NVSHMEMX_DT_FLOAT) nvshmem_float_put((float *)sym, (float *)src, len, q);
-          else nvshmem_double_put((double *)sym, (double *)src, len, q);
-        } else {
-          char *sym = c.arena + so + (unsigned long long)pe * bytes;
-          char *dst = slice_ptr(c, pe, ro + (unsigned long long)q * bytes);
-          if (dtype == NVSHMEMX_DT_INT) nvshmem_int_get((int *)dst, (int *)sym, len, q);
-          else if (dtype == NVSHMEMX_DT_FLOAT) nvshmem_float_get((float *)dst, (float *)sym, len, q);
-          else nvshmem_double_get((double *)dst, (double *)sym, len, q);
-        }
-      }
+      // the copies of nvshmem_{T}_put / _get by one thread per message; the
+      // lanes without a message help (copy_lanes)
+      char *dst = nullptr;
+      const char *src = nullptr;
+      const bool mine = unit < nunits;
+      if (mine) a2a_message(c, op, pe, so, ro, bytes, unit, &dst, &src);
+      const bool rec = mine && c.trace;
+      const unsigned long long t0 = rec ? gtimer() : 0;
+      copy_lanes<8, 4, true>(dst, src, mine ? bytes : 0);
+      if (rec)
+        trace_rec(c, (op == NVSHMEMX_REQ_PUT ? NVSHMEMX_TRACE_PUT_INT : NVSHMEMX_TRACE_GET_INT) + dtype,
+                  op == NVSHMEMX_REQ_PUT ? src : dst, op == NVSHMEMX_REQ_PUT ? dst : src, bytes,
+                  (pe + 1 + (int)unit) % np, t0, gtimer());
     } else if (MODE == NVSHMEMX_MODE_BULK && ((bytes | so | ro) & 15) == 0) {
       // one ring per CTA across its whole share of the round
       const unsigned long long seg = (((total + nunits - 1) / nunits) + 15) & ~15ull;
@@ -430,20 +453,24 @@ __global__ void alltoall_kernel(Cfg c, int op, int dtype, unsigned long long sen
       while (b < e) {
         const unsigned long long k = b / bytes, off = b - k * bytes;
         const unsigned long long len = (e - b) < (bytes - off) ? (e - b) : (bytes - off);
-        const int q = (pe + 1 + (int)k) % np;
-        if (op == NVSHMEMX_REQ_PUT) {
-          char *sym = c.arena + ro + (unsigned long long)pe * bytes + off;
-          char *src = slice_ptr(c, pe, so + (unsigned long long)q * bytes + off);
-          if (MODE == NVSHMEMX_MODE_WARP) nvshmemx_putmem_warp(sym, src, len, q);
-          else if (MODE == NVSHMEMX_MODE_BLOCK) nvshmemx_putmem_block(sym, src, len, q);
-          else nvshmemx_putmem_bulk_block(sym, src, len, q, smem, bulk_smem);
-        } else {
-          char *sym = c.arena + so + (unsigned long long)pe * bytes + off;
-          char *dst = slice_ptr(c, pe, ro + (unsigned long long)q * bytes + off);
-          if (MODE == NVSHMEMX_MODE_WARP) nvshmemx_getmem_warp(dst, sym, len, q);
-          else if (MODE == NVSHMEMX_MODE_BLOCK) nvshmemx_getmem_block(dst, sym, len, q);
-          else nvshmemx_getmem_bulk_block(dst, sym, len, q, smem, bulk_smem);
-        }
+        char *dst;
+        const char *src;
+        a2a_message(c, op, pe, so, ro, bytes, k, &dst, &src);
+        dst += off;
+        src += off;
+        const bool rec = c.trace && (MODE == NVSHMEMX_MODE_WARP ? (threadIdx.x & 31) == 0
+                                                                : MODE == NVSHMEMX_MODE_BLOCK && threadIdx.x == 0);
+        const unsigned long long t0 = rec ? gtimer() : 0;
+        if (MODE == NVSHMEMX_MODE_WARP)
+          copy_coop<16, 8, 4>(dst, src, len, threadIdx.x & 31, 32);
+        else if (MODE == NVSHMEMX_MODE_BLOCK)
+          copy_coop<16, 8>(dst, src, len, threadIdx.x, blockDim.x);
+        else
+          bulk_copy_block(c, dst, src, len, smem, bulk_smem);
+        if (rec)
+          trace_rec(c, op == NVSHMEMX_REQ_PUT ? NVSHMEMX_TRACE_PUT_INT : NVSHMEMX_TRACE_GET_INT,
+                    op == NVSHMEMX_REQ_PUT ? src : dst, op == NVSHMEMX_REQ_PUT ? dst : src, len,
+                    (pe + 1 + (int)k) % np, t0, gtimer());
         b += len;
       }
     }
@@ -481,7 +508,10 @@ __device__ __forceinline__ void halo_row_put(const Cfg &c, double *dst_sym, cons
   if (!check_remote(c, dst_sym, bytes, pe) || !check_local(c, src, bytes)) return;
   char *dst = xlate(c, dst_sym, pe);
   const unsigned long long t0 = (c.trace && lane == 0) ? gtimer() : 0;
-  copy_coop<16, 4>(dst, reinterpret_cast<const char *>(src), bytes, lane, 32);
+  if ((((uintptr_t)dst ^ (uintptr_t)src) & 15) == 0)
+    copy_body<16, 4>(dst, reinterpret_cast<const char *>(src), bytes, lane, 32);
+  else
+    copy_body<8, 4>(dst, reinterpret_cast<const char *>(src), bytes, lane, 32);
   if (c.trace && lane == 0) trace_rec(c, NVSHMEMX_TRACE_PUT_INT, src, dst, bytes, pe, t0, gtimer());
 }
 
@@ -663,10 +693,10 @@ int launch_exec_requests(int mode, const nvshmemx_request *dr, int n, cudaStream
   if (n <= 0) return 0;
   switch (mode) {
     case NVSHMEMX_MODE_THREAD:
-      exec_requests_kernel<NVSHMEMX_MODE_THREAD><<<(n + 255) / 256, 256, 0, s>>>(c, dr, n, 0);
+      exec_requests_kernel<NVSHMEMX_MODE_THREAD><<<(n + 63) / 64, 64, 0, s>>>(c, dr, n, 0);
       break;
     case NVSHMEMX_MODE_WARP:
-      exec_requests_kernel<NVSHMEMX_MODE_WARP><<<(n + 7) / 8, 256, 0, s>>>(c, dr, n, 0);
+      exec_requests_kernel<NVSHMEMX_MODE_WARP><<<(n + 1) / 2, 64, 0, s>>>(c, dr, n, 0);
       break;
     case NVSHMEMX_MODE_BLOCK:
       exec_requests_kernel<NVSHMEMX_MODE_BLOCK><<<n, 256, 0, s>>>(c, dr, n, 0);
