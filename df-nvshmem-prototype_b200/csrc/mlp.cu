@@ -3,19 +3,28 @@
 // and Adam kernels, and the executor of the 12 transfer variants it chooses
 // between.
 //
-// Kernel shape: one CTA of 64 threads per tile of 32 samples; all weights sit
-// in shared memory with rows padded by one float, so the forward pass (thread
-// = output unit, reading its weight row) and the backward pass (thread = input
-// unit, reading a weight column) are both free of bank conflicts.  Per-tile
-// weight gradients are summed over the tile's samples in registers and added
-// to the global gradient with one atomicAdd per weight per tile.  The network
-// is tiny (9,548 parameters); the work is latency-bound, not a contraction
-// worth the tensor cores.
+// Kernel shape: a CTA of 256 threads per tile of 16 rows, weights and
+// activations in shared memory.  Rows of 64 values lie 68 floats apart, so
+// the 16-byte reads of eight lanes (eight weight rows, or one row's
+// consecutive columns) fall into different banks.  The network is tiny (9,548
+// parameters), so it is bound by latency: shared-memory reads within a tile
+// (a 64 x 64 layer's weights are read once per row group) and
+// what has to be exchanged between tiles.  It stays in FP32 on the CUDA
+// cores: the tensor cores have no FP32 form, and a tile is 16 rows.
+//
+// Training is a chain of small steps, so it runs as one launch of one
+// thread-block cluster (train_cluster_kernel): the weights stay in shared
+// memory from step to step, the partial gradients are read by their owners
+// through distributed shared memory, and a step costs two cluster barriers
+// instead of three launches.  800 rows, batch 128: 75 us a step as a memset, a
+// gradient kernel (64 threads per 32 rows) and an Adam kernel, 12 us now, of
+// which the tile takes 5 us and the exchange of gradients and weights 6 us.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <string.h>
 
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "batch.h"
@@ -23,181 +32,485 @@
 
 namespace nvshm {
 
-constexpr int NI = NVSHMEMX_PICKER_NIN, NH = NVSHMEMX_PICKER_HIDDEN, NO = NVSHMEMX_PICKER_VARIANTS, TS = 32;
+constexpr int NI = NVSHMEMX_PICKER_NIN, NH = NVSHMEMX_PICKER_HIDDEN, NO = NVSHMEMX_PICKER_VARIANTS;
 constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + NH * NI, OFF_W2 = OFF_B1 + NH, OFF_B2 = OFF_W2 + NH * NH,
               OFF_W3 = OFF_B2 + NH, OFF_B3 = OFF_W3 + NH * NH, OFF_W4 = OFF_B3 + NH, OFF_B4 = OFF_W4 + NO * NH,
               NPARAM = OFF_B4 + NO;
-// shared-memory floats: padded weights, biases, inputs, three activations,
-// outputs, two gradient buffers
-constexpr int SM_FLOATS = NH * (NI + 1) + 2 * NH * (NH + 1) + NO * (NH + 1) + 3 * NH + 16 + TS * NI + 3 * TS * NH +
-                          TS * NO + 2 * TS * NH;
+constexpr int kThreads = 256;
+constexpr int kRows = 16;       // rows of a tile of the grid kernels
+constexpr int kTrainRows = 8;   // rows of a CTA's tile in a training cluster
+constexpr int LD = NH + 4;  // floats between rows of 64
+constexpr int LDX = 12;     // floats between rows of 6 (padded with zeros to 8)
+static_assert(NI <= 8 && NH == 64 && NO == 12, "the thread mappings below are for these sizes");
 
-template <bool BWD>
-__global__ void __launch_bounds__(64) mlp_kernel(const float *__restrict__ P, const float *__restrict__ X,
-                                                 const float *__restrict__ Y, const float *__restrict__ M,
-                                                 const int *__restrict__ idx, int n, const float *__restrict__ norm,
-                                                 float inv_count, float *__restrict__ out, float *__restrict__ grad,
-                                                 float *__restrict__ loss) {
-  extern __shared__ float sm[];
-  float *W1 = sm;
-  float *W2 = W1 + NH * (NI + 1);
-  float *W3 = W2 + NH * (NH + 1);
-  float *W4 = W3 + NH * (NH + 1);
-  float *b1 = W4 + NO * (NH + 1);
-  float *b2 = b1 + NH;
-  float *b3 = b2 + NH;
-  float *b4 = b3 + NH;
-  float *Xs = b4 + 16;
-  float *A1 = Xs + TS * NI;
-  float *A2 = A1 + TS * NH;
-  float *A3 = A2 + TS * NH;
-  float *Os = A3 + TS * NH;
-  float *dZ = Os + TS * NO;
-  float *dA = dZ + TS * NH;
+// Shared memory in floats.
+template <int R>
+struct Net {
+  float W1[NH * LDX], W2[NH * LD], W3[NH * LD], W4[NO * LD];
+  float b1[NH], b2[NH], b3[NH], b4[16];
+  float X[R * LDX];
+  float A1[R * LD], A2[R * LD], A3[R * LD];
+  float O[R * 16];  // outputs, then dL/dO
+};
+template <int R>
+struct NetGrad : Net<R> {
+  float Y[R * NO], M[R * NO];
+  float D1[R * LD], D2[R * LD], D3[R * LD];  // dL/dz of the hidden layers
+  float G[NPARAM + 4];                                   // gradient, in the parameters' own order
+  float loss;
+};
+
+// Where parameter p lies in the net's shared memory, in floats from its start.
+__host__ __device__ __forceinline__ int param_slot(int p) {
+  constexpr int sW2 = NH * LDX, sW3 = sW2 + NH * LD, sW4 = sW3 + NH * LD, sb1 = sW4 + NO * LD, sb2 = sb1 + NH,
+                sb3 = sb2 + NH, sb4 = sb3 + NH;
+  if (p < OFF_B1) return (p / NI) * LDX + p % NI;
+  if (p < OFF_W2) return sb1 + (p - OFF_B1);
+  if (p < OFF_B2) return sW2 + ((p - OFF_W2) / NH) * LD + (p - OFF_W2) % NH;
+  if (p < OFF_W3) return sb2 + (p - OFF_B2);
+  if (p < OFF_B3) return sW3 + ((p - OFF_W3) / NH) * LD + (p - OFF_W3) % NH;
+  if (p < OFF_W4) return sb3 + (p - OFF_B3);
+  if (p < OFF_B4) return sW4 + ((p - OFF_W4) / NH) * LD + (p - OFF_W4) % NH;
+  return sb4 + (p - OFF_B4);
+}
+
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+
+template <int R>
+__device__ __forceinline__ void load_net(Net<R> &s, const float *__restrict__ P) {
   const int t = threadIdx.x;
-  for (int i = t; i < NH * NI; i += 64) W1[(i / NI) * (NI + 1) + i % NI] = P[OFF_W1 + i];
-  for (int i = t; i < NH * NH; i += 64) {
-    W2[(i / NH) * (NH + 1) + i % NH] = P[OFF_W2 + i];
-    W3[(i / NH) * (NH + 1) + i % NH] = P[OFF_W3 + i];
-  }
-  for (int i = t; i < NO * NH; i += 64) W4[(i / NH) * (NH + 1) + i % NH] = P[OFF_W4 + i];
-  b1[t] = P[OFF_B1 + t];
-  b2[t] = P[OFF_B2 + t];
-  b3[t] = P[OFF_B3 + t];
-  if (t < NO) b4[t] = P[OFF_B4 + t];
-  const int s0 = blockIdx.x * TS;
-  const int ns = min(TS, n - s0);
-  for (int i = t; i < TS * NI; i += 64) {
-    const int s = i / NI, f = i % NI;
-    float v = 0.f;
-    if (s < ns) {
-      const int g = idx ? idx[s0 + s] : s0 + s;
-      v = (X[g * NI + f] - norm[f]) / norm[NI + f];
-    }
-    Xs[i] = v;
-  }
+  for (int i = t; i < NH * LDX; i += kThreads) s.W1[i] = 0.f;
+  for (int i = t; i < R * LDX; i += kThreads) s.X[i] = 0.f;
   __syncthreads();
-  // forward: thread t is output unit t
-  for (int s = 0; s < TS; ++s) {
-    float a = b1[t];
+  float *base = s.W1;
+  for (int p = t; p < NPARAM; p += kThreads) base[param_slot(p)] = P[p];
+}
+
+// out[r][j] = relu(b[j] + sum_k W[j][k] in[r][k]): a warp takes 32 outputs
+// (one per lane) of R / 4 rows.
+template <int R, int K4>
+__device__ __forceinline__ void forward_layer(const float *W, int ldw, const float *b, const float *in, int ldin,
+                                              float *out) {
+  constexpr int N = R / 4;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int j = (w & 1) * 32 + lane, r0 = (w >> 1) * N;
+  float a[N];
 #pragma unroll
-    for (int i = 0; i < NI; ++i) a += W1[t * (NI + 1) + i] * Xs[s * NI + i];
-    A1[s * NH + t] = fmaxf(a, 0.f);
-  }
-  __syncthreads();
-  for (int s = 0; s < TS; ++s) {
-    float a = b2[t];
-    for (int i = 0; i < NH; ++i) a += W2[t * (NH + 1) + i] * A1[s * NH + i];
-    A2[s * NH + t] = fmaxf(a, 0.f);
-  }
-  __syncthreads();
-  for (int s = 0; s < TS; ++s) {
-    float a = b3[t];
-    for (int i = 0; i < NH; ++i) a += W3[t * (NH + 1) + i] * A2[s * NH + i];
-    A3[s * NH + t] = fmaxf(a, 0.f);
-  }
-  __syncthreads();
-  if (t < NO) {
-    for (int s = 0; s < TS; ++s) {
-      float a = b4[t];
-      for (int i = 0; i < NH; ++i) a += W4[t * (NH + 1) + i] * A3[s * NH + i];
-      Os[s * NO + t] = a;
+  for (int r = 0; r < N; ++r) a[r] = b[j];
+#pragma unroll 8
+  for (int k = 0; k < K4; ++k) {
+    const float4 x = ld4(W + j * ldw + 4 * k);
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+      const float4 y = ld4(in + (r0 + r) * ldin + 4 * k);
+      a[r] += x.x * y.x;
+      a[r] += x.y * y.y;
+      a[r] += x.z * y.z;
+      a[r] += x.w * y.w;
     }
   }
-  __syncthreads();
-  if (!BWD) {
-    for (int i = t; i < ns * NO; i += 64) out[(size_t)(s0 + i / NO) * NO + i % NO] = Os[i];
-    return;
+#pragma unroll
+  for (int r = 0; r < N; ++r) out[(r0 + r) * LD + j] = fmaxf(a[r], 0.f);
+}
+
+// The outputs of a warp's R / 8 rows, one per lane.
+template <int R>
+__device__ __forceinline__ bool output_of(int *row, int *k) {
+  const int lane = threadIdx.x & 31;
+  *row = (threadIdx.x >> 5) * (R / 8) + lane / NO;
+  *k = lane % NO;
+  return lane < R / 8 * NO;
+}
+template <int R>
+__device__ __forceinline__ float output_value(const Net<R> &s, int row, int k) {
+  float a = s.b4[k];
+#pragma unroll 8
+  for (int i = 0; i < NH; i += 4) {
+    const float4 x = ld4(s.W4 + k * LD + i), y = ld4(s.A3 + row * LD + i);
+    a += x.x * y.x;
+    a += x.y * y.y;
+    a += x.z * y.z;
+    a += x.w * y.w;
   }
-  // loss and dL/dO = 2 m (o - y) / count, in place
-  float lsum = 0.f;
-  for (int i = t; i < TS * NO; i += 64) {
-    const int s = i / NO, k = i % NO;
+  return a;
+}
+
+// Hidden layers of the tile in s.X; ends with a barrier.
+template <int R>
+__device__ __forceinline__ void forward_hidden(Net<R> &s) {
+  forward_layer<R, 2>(s.W1, LDX, s.b1, s.X, LDX, s.A1);
+  __syncthreads();
+  forward_layer<R, 16>(s.W2, LD, s.b2, s.A1, LD, s.A2);
+  __syncthreads();
+  forward_layer<R, 16>(s.W3, LD, s.b3, s.A2, LD, s.A3);
+  __syncthreads();
+}
+
+__device__ __forceinline__ void put_grad(float *g, float v, bool first) { *g = first ? v : *g + v; }
+__device__ __forceinline__ void put_grad4(float *g, const float *v, bool first) {
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (!first) o = ld4(g);
+  *reinterpret_cast<float4 *>(g) = make_float4(o.x + v[0], o.y + v[1], o.z + v[2], o.w + v[3]);
+}
+
+// G += D^T A (64 x 64) and its bias gradient: a 4 x 4 block per thread.
+template <int R>
+__device__ __forceinline__ void weight_grad(const float *D, const float *A, float *gw, float *gb, bool first) {
+  const int i4 = (threadIdx.x & 15) * 4, j4 = (threadIdx.x >> 4) * 4;
+  float g[4][4] = {}, sb[4] = {};
+#pragma unroll 4
+  for (int r = 0; r < R; ++r) {
+    const float4 d = ld4(D + r * LD + j4), a = ld4(A + r * LD + i4);
+    const float dv[4] = {d.x, d.y, d.z, d.w}, av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      sb[j] += dv[j];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g[j][i] += dv[j] * av[i];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) put_grad4(gw + (j4 + j) * NH + i4, g[j], first);
+  if (i4 == 0) put_grad4(gb + j4, sb, first);
+}
+
+// out = (D W) where A > 0: R / 8 rows per warp, half of the sum per half
+// warp, four columns per lane.
+template <int R>
+__device__ __forceinline__ void input_grad(const float *D, const float *W, const float *A, float *out) {
+  constexpr int N = R / 8;
+  const int lane = threadIdx.x & 31, i4 = (lane & 15) * 4, half = lane >> 4, r0 = (threadIdx.x >> 5) * N;
+  float a[N][4] = {};
+#pragma unroll 4
+  for (int j = half * 32; j < half * 32 + 32; j += 4) {
+    float e[N][4];
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+      const float4 d = ld4(D + (r0 + r) * LD + j);
+      e[r][0] = d.x, e[r][1] = d.y, e[r][2] = d.z, e[r][3] = d.w;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float4 w = ld4(W + (j + u) * LD + i4);
+      const float wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int r = 0; r < N; ++r)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[r][i] += e[r][u] * wv[i];
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < N; ++r)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[r][i] += __shfl_xor_sync(0xffffffffu, a[r][i], 16);
+  // both halves hold every sum: of two rows each writes one, of one row the
+  // first writes it
+  const int r = N == 2 ? half : 0;
+  if (N == 2 || half == 0) {
+    const float *m = A + (r0 + r) * LD + i4;
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = m[i] > 0.f ? a[N == 2 && half ? N - 1 : 0][i] : 0.f;
+    *reinterpret_cast<float4 *>(out + (r0 + r) * LD + i4) = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+
+// Forward and backward of the tile in s.X, s.Y, s.M (`rows` valid rows):
+// adds its loss to s.loss and its gradient to s.G (`first`: replaces it).
+// Begins and ends with every thread past a barrier for the inputs / not yet
+// past one for s.G.
+template <int R>
+__device__ __forceinline__ void tile_gradient(NetGrad<R> &s, int rows, float inv_count, bool first) {
+  const int t = threadIdx.x;
+  forward_hidden(s);
+  int row, k;
+  float l = 0.f;
+  if (output_of<R>(&row, &k)) {
     float d = 0.f;
-    if (s < ns) {
-      const int g = idx ? idx[s0 + s] : s0 + s;
-      const float m = M[g * NO + k], diff = Os[i] - Y[g * NO + k];
+    if (row < rows) {
+      const float m = s.M[row * NO + k], diff = output_value(s, row, k) - s.Y[row * NO + k];
       d = 2.f * m * diff * inv_count;
-      lsum += m * diff * diff;
+      l = m * diff * diff;
     }
-    Os[i] = d;
+    s.O[row * 16 + k] = d;
   }
-  for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if ((t & 31) == 0) atomicAdd(loss, lsum * inv_count);
+  for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+  if ((t & 31) == 0) atomicAdd(&s.loss, l * inv_count);
   __syncthreads();
-  // layer 4: thread t is input column t
-  for (int k = 0; k < NO; ++k) {
-    float acc = 0.f;
-    for (int s = 0; s < TS; ++s) acc += Os[s * NO + k] * A3[s * NH + t];
-    atomicAdd(&grad[OFF_W4 + k * NH + t], acc);
+  // layer 4: four columns of one output per thread; the output's bias
+  if (t < NO * 16) {
+    const int q = t >> 4, i4 = (t & 15) * 4;
+    float g[4] = {};
+#pragma unroll 4
+    for (int r = 0; r < R; ++r) {
+      const float d = s.O[r * 16 + q];
+      const float4 a = ld4(s.A3 + r * LD + i4);
+      g[0] += d * a.x;
+      g[1] += d * a.y;
+      g[2] += d * a.z;
+      g[3] += d * a.w;
+    }
+    put_grad4(s.G + OFF_W4 + q * NH + i4, g, first);
+  } else if (t < NO * 16 + NO) {
+    float g = 0.f;
+    for (int r = 0; r < R; ++r) g += s.O[r * 16 + (t - NO * 16)];
+    put_grad(s.G + OFF_B4 + (t - NO * 16), g, first);
   }
-  if (t < NO) {
-    float acc = 0.f;
-    for (int s = 0; s < TS; ++s) acc += Os[s * NO + t];
-    atomicAdd(&grad[OFF_B4 + t], acc);
-  }
-  for (int s = 0; s < TS; ++s) {
-    float acc = 0.f;
-    for (int k = 0; k < NO; ++k) acc += Os[s * NO + k] * W4[k * (NH + 1) + t];
-    dZ[s * NH + t] = A3[s * NH + t] > 0.f ? acc : 0.f;
+  if (t < R * 16) {
+    const int r = t >> 4, i4 = (t & 15) * 4;
+    float a[4] = {};
+#pragma unroll
+    for (int q = 0; q < NO; ++q) {
+      const float d = s.O[r * 16 + q];
+      const float4 w = ld4(s.W4 + q * LD + i4);
+      a[0] += d * w.x;
+      a[1] += d * w.y;
+      a[2] += d * w.z;
+      a[3] += d * w.w;
+    }
+    const float4 m = ld4(s.A3 + r * LD + i4);
+    *reinterpret_cast<float4 *>(s.D3 + r * LD + i4) = make_float4(
+        m.x > 0.f ? a[0] : 0.f, m.y > 0.f ? a[1] : 0.f, m.z > 0.f ? a[2] : 0.f, m.w > 0.f ? a[3] : 0.f);
   }
   __syncthreads();
-  // layer 3 (dZ holds dL/dz3)
-  for (int j = 0; j < NH; ++j) {
-    float acc = 0.f;
-    for (int s = 0; s < TS; ++s) acc += dZ[s * NH + j] * A2[s * NH + t];
-    atomicAdd(&grad[OFF_W3 + j * NH + t], acc);
-  }
+  weight_grad<R>(s.D3, s.A2, s.G + OFF_W3, s.G + OFF_B3, first);
+  input_grad<R>(s.D3, s.W3, s.A2, s.D2);
+  __syncthreads();
+  weight_grad<R>(s.D2, s.A1, s.G + OFF_W2, s.G + OFF_B2, first);
+  input_grad<R>(s.D2, s.W2, s.A1, s.D1);
+  __syncthreads();
+  // layer 1: one output's inputs f and f + 4 per thread; the bias where
+  // there is no f + 4 within the six
   {
-    float acc = 0.f;
-    for (int s = 0; s < TS; ++s) acc += dZ[s * NH + t];
-    atomicAdd(&grad[OFF_B3 + t], acc);
+    const int j = t & 63, f = t >> 6;
+    float g0 = 0.f, g1 = 0.f, sb = 0.f;
+    for (int r = 0; r < R; ++r) {
+      const float d = s.D1[r * LD + j];
+      g0 += d * s.X[r * LDX + f];
+      if (f + 4 < NI) g1 += d * s.X[r * LDX + f + 4];
+      sb += d;
+    }
+    put_grad(s.G + OFF_W1 + j * NI + f, g0, first);
+    if (f + 4 < NI) put_grad(s.G + OFF_W1 + j * NI + f + 4, g1, first);
+    if (f == 3) put_grad(s.G + OFF_B1 + j, sb, first);
   }
-  for (int s = 0; s < TS; ++s) {
-    float acc = 0.f;
-    for (int j = 0; j < NH; ++j) acc += dZ[s * NH + j] * W3[j * (NH + 1) + t];
-    dA[s * NH + t] = A2[s * NH + t] > 0.f ? acc : 0.f;
+}
+
+__device__ __forceinline__ float adam_step(float p, float g, float *m, float *v, float lr, float c1, float c2) {
+  const float mi = 0.9f * *m + 0.1f * g;
+  const float vi = 0.999f * *v + 0.001f * g * g;
+  *m = mi;
+  *v = vi;
+  return p - lr * (mi / c1) / (sqrtf(vi / c2) + 1e-8f);
+}
+
+// Y[n][12] of X[n][6], 16 rows at a time per CTA.
+__global__ void __launch_bounds__(kThreads) mlp_forward_kernel(const float *__restrict__ P, const float *__restrict__ X,
+                                                               int n, const float *__restrict__ norm,
+                                                               float *__restrict__ out) {
+  extern __shared__ __align__(16) char sm[];
+  Net<kRows> &s = *reinterpret_cast<Net<kRows> *>(sm);
+  load_net(s, P);
+  for (long long s0 = (long long)blockIdx.x * kRows; s0 < n; s0 += (long long)gridDim.x * kRows) {
+    __syncthreads();
+    if (threadIdx.x < kRows * NI) {
+      const int r = threadIdx.x / NI, f = threadIdx.x % NI;
+      s.X[r * LDX + f] = s0 + r < n ? (X[(s0 + r) * NI + f] - norm[f]) / norm[NI + f] : 0.f;
+    }
+    __syncthreads();
+    forward_hidden(s);
+    int row, k;
+    if (output_of<kRows>(&row, &k) && s0 + row < n) out[(s0 + row) * NO + k] = output_value(s, row, k);
+  }
+}
+
+// Loss and gradient of n rows (rows idx[0..n) when idx is given), added to
+// *loss and grad: every CTA sums its tiles in shared memory and adds them once.
+__global__ void __launch_bounds__(kThreads) mlp_grad_kernel(const float *__restrict__ P, const float *__restrict__ X,
+                                                            const float *__restrict__ Y, const float *__restrict__ M,
+                                                            const int *__restrict__ idx, int n,
+                                                            const float *__restrict__ norm, float inv_count,
+                                                            float *__restrict__ grad, float *__restrict__ loss) {
+  extern __shared__ __align__(16) char sm[];
+  NetGrad<kRows> &s = *reinterpret_cast<NetGrad<kRows> *>(sm);
+  const int t = threadIdx.x;
+  load_net(s, P);
+  if (t == 0) s.loss = 0.f;
+  bool first = true;
+  for (long long s0 = (long long)blockIdx.x * kRows; s0 < n; s0 += (long long)gridDim.x * kRows) {
+    const int rows = n - s0 < kRows ? (int)(n - s0) : kRows;
+    __syncthreads();
+    if (t < kRows * NO) {
+      const int r = t / NO, k = t % NO;
+      const long long g = r < rows ? (idx ? idx[s0 + r] : s0 + r) : 0;
+      s.Y[t] = r < rows ? Y[g * NO + k] : 0.f;
+      s.M[t] = r < rows ? M[g * NO + k] : 0.f;
+    }
+    if (t < kRows * NI) {
+      const int r = t / NI, f = t % NI;
+      const long long g = r < rows ? (idx ? idx[s0 + r] : s0 + r) : 0;
+      s.X[r * LDX + f] = r < rows ? (X[g * NI + f] - norm[f]) / norm[NI + f] : 0.f;
+    }
+    __syncthreads();
+    tile_gradient(s, rows, inv_count, first);
+    first = false;
   }
   __syncthreads();
-  // layer 2 (dA holds dL/dz2)
-  for (int j = 0; j < NH; ++j) {
-    float acc = 0.f;
-    for (int s = 0; s < TS; ++s) acc += dA[s * NH + j] * A1[s * NH + t];
-    atomicAdd(&grad[OFF_W2 + j * NH + t], acc);
-  }
-  {
-    float acc = 0.f;
-    for (int s = 0; s < TS; ++s) acc += dA[s * NH + t];
-    atomicAdd(&grad[OFF_B2 + t], acc);
-  }
-  for (int s = 0; s < TS; ++s) {
-    float acc = 0.f;
-    for (int j = 0; j < NH; ++j) acc += dA[s * NH + j] * W2[j * (NH + 1) + t];
-    dZ[s * NH + t] = A1[s * NH + t] > 0.f ? acc : 0.f;
-  }
-  __syncthreads();
-  // layer 1 (dZ holds dL/dz1): thread t is output unit t
-  for (int f = 0; f < NI; ++f) {
-    float acc = 0.f;
-    for (int s = 0; s < TS; ++s) acc += dZ[s * NH + t] * Xs[s * NI + f];
-    atomicAdd(&grad[OFF_W1 + t * NI + f], acc);
-  }
-  {
-    float acc = 0.f;
-    for (int s = 0; s < TS; ++s) acc += dZ[s * NH + t];
-    atomicAdd(&grad[OFF_B1 + t], acc);
-  }
+  if (first) return;
+  for (int p = t; p < NPARAM; p += kThreads) atomicAdd(&grad[p], s.G[p]);
+  if (t == 0) atomicAdd(loss, s.loss);
 }
 
 __global__ void adam_kernel(float *P, const float *G, float *m, float *v, int n, float lr, float c1, float c2) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float g = G[i];
-  const float mi = 0.9f * m[i] + 0.1f * g;
-  const float vi = 0.999f * v[i] + 0.001f * g * g;
-  m[i] = mi;
-  v[i] = vi;
-  P[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + 1e-8f);
+  if (i < n) P[i] = adam_step(P[i], G[i], m + i, v + i, lr, c1, c2);
+}
+
+// ------------------------------------------------ training in one cluster
+// One tile of a training run: up to 8 rows for each CTA of the cluster.
+struct TrainTile {
+  int first, rows;   // rows idx[first .. first + rows)
+  float inv_count;   // 1 / mask sum of its batch
+  float c1, c2;      // Adam's bias corrections of its batch's step
+  int flags;         // kFirst: begins a batch; kLast: ends it
+  int epoch;
+  int pad;
+};
+enum { kFirst = 1, kLast = 2 };
+constexpr int kCluster = 16;                                          // CTAs (8 took 14.4 us a step, 16 12.0 us)
+constexpr int kTileRows = kCluster * kTrainRows;                           // rows of a tile
+constexpr int kOwned = (NPARAM + kCluster - 1) / kCluster;              // parameters a CTA updates ...
+constexpr int kPerThread = (kOwned + kThreads - 1) / kThreads;          // ... and a thread of it
+// A batch of more rows is spread over more SMs than a cluster has: 512 rows
+// take the cluster 39 us a step, the three launches of a spread-out step 37 us;
+// 256 rows 22 us.
+constexpr int kClusterBatch = 512;
+
+__device__ __forceinline__ unsigned peer_addr(const void *p, unsigned rank) {
+  unsigned a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float ld_peer(unsigned a) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_peer(unsigned a, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Every CTA holds the whole network and takes 8 of a tile's 128 rows.  After
+// a batch's last tile, CTA c sums the cluster's gradients of parameters
+// [c * kOwned, (c + 1) * kOwned) in rank order (so training is reproducible),
+// updates them (their moments stay in its registers) and writes the new
+// values into every CTA's network.  The next tile's rows, and the row numbers
+// of the one after, are fetched while a tile is computed.
+__global__ void __launch_bounds__(kThreads) train_cluster_kernel(float *__restrict__ P, float *__restrict__ Am,
+                                                                 float *__restrict__ Av, const float *__restrict__ X,
+                                                                 const float *__restrict__ Y,
+                                                                 const float *__restrict__ M,
+                                                                 const int *__restrict__ idx,
+                                                                 const TrainTile *__restrict__ tiles, int ntiles,
+                                                                 const float *__restrict__ norm, float lr,
+                                                                 float *__restrict__ losses) {
+  extern __shared__ __align__(16) char sm[];
+  NetGrad<kTrainRows> &s = *reinterpret_cast<NetGrad<kTrainRows> *>(sm);
+  const int t = threadIdx.x, rank = blockIdx.x;
+  load_net(s, P);
+  if (t == 0) s.loss = 0.f;
+  float p[kPerThread], m[kPerThread], v[kPerThread];
+#pragma unroll
+  for (int i = 0; i < kPerThread; ++i) {
+    const int q = t + i * kThreads, g = rank * kOwned + q;
+    const bool own = q < kOwned && g < NPARAM;
+    p[i] = own ? P[g] : 0.f;
+    m[i] = own ? Am[g] : 0.f;
+    v[i] = own ? Av[g] : 0.f;
+  }
+  int slot[kPerThread];
+#pragma unroll
+  for (int i = 0; i < kPerThread; ++i) {
+    const int g = rank * kOwned + t + i * kThreads;
+    slot[i] = param_slot(g < NPARAM ? g : 0);
+  }
+  // this thread's part of a tile: one output of one row, one input of one row
+  const int yr = t / NO, yk = t % NO, xr = t / NI, xf = t % NI;
+  const bool has_y = t < kTrainRows * NO, has_x = t < kTrainRows * NI;
+  const float mean = has_x ? norm[xf] : 0.f, sd = has_x ? norm[NI + xf] : 1.f;
+  auto row_of = [&](const TrainTile &d, int r) { return rank * kTrainRows + r < d.rows ? idx[d.first + rank * kTrainRows + r] : -1; };
+  TrainTile cur = tiles[0], nxt = tiles[ntiles > 1 ? 1 : 0];
+  int gy = has_y ? row_of(cur, yr) : -1, gx = has_x ? row_of(cur, xr) : -1;
+  float y = gy >= 0 ? Y[(size_t)gy * NO + yk] : 0.f, mk = gy >= 0 ? M[(size_t)gy * NO + yk] : 0.f;
+  float x = gx >= 0 ? X[(size_t)gx * NI + xf] : 0.f;
+  int ny = has_y ? row_of(nxt, yr) : -1, nx = has_x ? row_of(nxt, xr) : -1;
+  float epoch_loss = 0.f;  // rank 0, thread 0
+  cluster_barrier();
+  for (int i = 0; i < ntiles; ++i) {
+    if (has_y) {
+      s.Y[t] = y;
+      s.M[t] = mk;
+    }
+    if (has_x) s.X[xr * LDX + xf] = gx >= 0 ? (x - mean) / sd : 0.f;
+    __syncthreads();
+    const TrainTile d = cur;
+    const TrainTile after = tiles[i + 2 < ntiles ? i + 2 : ntiles - 1];
+    y = ny >= 0 ? Y[(size_t)ny * NO + yk] : 0.f;
+    mk = ny >= 0 ? M[(size_t)ny * NO + yk] : 0.f;
+    x = nx >= 0 ? X[(size_t)nx * NI + xf] : 0.f;
+    gx = nx;
+    cur = nxt;
+    nxt = after;
+    ny = has_y ? row_of(after, yr) : -1;
+    nx = has_x ? row_of(after, xr) : -1;
+    int rows = d.rows - rank * kTrainRows;
+    rows = rows < 0 ? 0 : (rows > kTrainRows ? kTrainRows : rows);
+    tile_gradient(s, rows, d.inv_count, (d.flags & kFirst) != 0);
+    if (!(d.flags & kLast)) {
+      __syncthreads();
+      continue;
+    }
+    cluster_barrier();  // every CTA's gradient and loss of the batch are there
+    if (rank == 0 && t == 0) {
+      float l = 0.f;
+      for (unsigned r = 0; r < kCluster; ++r) l += ld_peer(peer_addr(&s.loss, r));
+      epoch_loss += l;
+      if (i + 1 == ntiles || cur.epoch != d.epoch) {
+        losses[d.epoch] = epoch_loss;
+        epoch_loss = 0.f;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kPerThread; ++k) {
+      const int q = t + k * kThreads, g = rank * kOwned + q;
+      if (q < kOwned && g < NPARAM) {
+        float part[kCluster];
+#pragma unroll
+        for (unsigned r = 0; r < kCluster; ++r) part[r] = ld_peer(peer_addr(s.G + g, r));
+        float sum = part[0];
+#pragma unroll
+        for (int r = 1; r < kCluster; ++r) sum += part[r];
+        p[k] = adam_step(p[k], sum, &m[k], &v[k], lr, d.c1, d.c2);
+#pragma unroll
+        for (unsigned r = 0; r < kCluster; ++r) st_peer(peer_addr(s.W1 + slot[k], r), p[k]);
+      }
+    }
+    cluster_barrier();  // the new weights are everywhere, nobody reads G or loss any more
+    if (t == 0) s.loss = 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < kPerThread; ++i) {
+    const int q = t + i * kThreads, g = rank * kOwned + q;
+    if (q < kOwned && g < NPARAM) {
+      P[g] = p[i];
+      Am[g] = m[i];
+      Av[g] = v[i];
+    }
+  }
 }
 
 // Deterministic host RNG for initialisation and shuffles.
@@ -212,38 +525,152 @@ static unsigned long long mix64(unsigned long long x) {
 
 using namespace nvshm;
 
-struct nvshmemx_mlp {
-  float *P = nullptr, *G = nullptr, *Am = nullptr, *Av = nullptr;  // params, grad, Adam moments
-  float *norm = nullptr;                                           // mean[6], std[6]
-  float *loss = nullptr;
-  long long step = 0;
-};
+// Memory of a network: its own arrays and kSlotWork bytes for the host arrays
+// of a call.  The first kSlots networks of a device live in an array of the
+// library (the device's allocator takes 0.3-0.6 ms to map a first block and
+// as long to give it back, several times what training a table of 800
+// classes for some epochs takes); further ones are allocated.
+constexpr size_t pad256(size_t x) { return (x + 255) / 256 * 256; }
+constexpr size_t kParBytes = pad256(NPARAM * 4), kNormBytes = pad256(2 * NI * 4);
+constexpr size_t kNetBytes = 4 * kParBytes + kNormBytes + 256, kSlotWork = 256u << 10;
+constexpr int kSlots = 2, kMaxDevices = 64;
+static __device__ __align__(256) unsigned char g_mlp_slots[kSlots][kNetBytes + kSlotWork];
+static std::mutex g_slot_mu;
+static bool g_slot_used[kMaxDevices][kSlots];
 
-static int mlp_launch(nvshmemx_mlp *m, bool bwd, const float *dX, const float *dY, const float *dM, const int *didx,
-                      int n, float inv_count, float *dout) {
-  const size_t smem = (size_t)SM_FLOATS * sizeof(float);
-  const void *fn = bwd ? (const void *)mlp_kernel<true> : (const void *)mlp_kernel<false>;
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const int blocks = (n + TS - 1) / TS;
-  if (bwd)
-    mlp_kernel<true><<<blocks, 64, smem>>>(m->P, dX, dY, dM, didx, n, m->norm, inv_count, dout, m->G, m->loss);
-  else
-    mlp_kernel<false><<<blocks, 64, smem>>>(m->P, dX, dY, dM, didx, n, m->norm, inv_count, dout, m->G, m->loss);
-  return check_cuda(cudaGetLastError(), "mlp kernel");
+// Takes a free slot of device `dev` (the current one): its number and address,
+// or -1.
+static int take_slot(int dev, char **p) {
+  if (dev < 0 || dev >= kMaxDevices) return -1;
+  std::lock_guard<std::mutex> lk(g_slot_mu);
+  for (int k = 0; k < kSlots; ++k) {
+    if (g_slot_used[dev][k]) continue;
+    void *base = nullptr;
+    if (cudaGetSymbolAddress(&base, g_mlp_slots) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return -1;
+    }
+    g_slot_used[dev][k] = true;
+    *p = (char *)base + k * (kNetBytes + kSlotWork);
+    return k;
+  }
+  return -1;
 }
 
-struct DevArr {
-  void *p = nullptr;
-  ~DevArr() {
-    if (p) cudaFree(p);
+static void give_slot(int dev, int k) {
+  std::lock_guard<std::mutex> lk(g_slot_mu);
+  g_slot_used[dev][k] = false;
+}
+
+struct nvshmemx_mlp {
+  char *block = nullptr;  // everything below in one allocation
+  float *P = nullptr, *norm = nullptr, *Am = nullptr, *Av = nullptr, *G = nullptr, *loss = nullptr;
+  long long step = 0;
+  int sms = 0;
+  int cluster = -1;  // whether a training cluster fits the device (-1: not asked yet)
+  int dev = 0, slot = -1;
+  // Device copies of the host arrays of a call, kept between calls up to
+  // kKeep bytes; a larger call allocates its own.  `mu` holds a call's use of
+  // them (and of G and loss), so calls on one network from several threads
+  // run one after the other.
+  std::mutex mu;
+  char *work = nullptr;
+  size_t work_bytes = 0;
+  bool work_own = false;  // allocated (else part of a slot)
+};
+
+static const size_t kKeep = 16u << 20;
+
+// Device memory for one call, held under the network's lock.
+struct Work {
+  std::lock_guard<std::mutex> lk;
+  char *p = nullptr;
+  char *own = nullptr;
+  explicit Work(nvshmemx_mlp *m) : lk(m->mu) {}
+  ~Work() {
+    if (own) cudaFree(own);
+  }
+  int get(nvshmemx_mlp *m, size_t bytes) {
+    if (bytes > kKeep) {
+      if (cudaMalloc(&own, bytes) != cudaSuccess) return fail(NVSHMEMX_ERR_NOMEM, "mlp: cudaMalloc");
+      p = own;
+      return 0;
+    }
+    if (bytes > m->work_bytes) {
+      size_t want = 64u << 10;
+      while (want < bytes) want *= 2;
+      if (m->work_own) cudaFree(m->work);
+      m->work = nullptr;
+      m->work_bytes = 0;
+      m->work_own = false;
+      if (cudaMalloc(&m->work, want) != cudaSuccess) return fail(NVSHMEMX_ERR_NOMEM, "mlp: cudaMalloc");
+      m->work_own = true;
+      m->work_bytes = want;
+    }
+    p = m->work;
+    return 0;
   }
 };
 
-// Device copy of a host array; h == nullptr only allocates (an output).
-static int upload(DevArr &a, const void *h, size_t bytes) {
-  if (cudaMalloc(&a.p, bytes ? bytes : 4) != cudaSuccess) return fail(NVSHMEMX_ERR_NOMEM, "mlp: cudaMalloc");
-  if (bytes && h) return check_cuda(cudaMemcpy(a.p, h, bytes, cudaMemcpyHostToDevice), "mlp: upload");
-  return 0;
+static int upload(void *d, const void *h, size_t bytes) {
+  return bytes ? check_cuda(cudaMemcpy(d, h, bytes, cudaMemcpyHostToDevice), "mlp: upload") : 0;
+}
+
+static int launch_forward(nvshmemx_mlp *m, const float *dX, int n, float *dY) {
+  cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Net<kRows>));
+  const int blocks = std::min((n - 1) / kRows + 1, 3 * m->sms);
+  mlp_forward_kernel<<<blocks, kThreads, sizeof(Net<kRows>)>>>(m->P, dX, n, m->norm, dY);
+  return check_cuda(cudaGetLastError(), "mlp forward kernel");
+}
+
+static int launch_grad(nvshmemx_mlp *m, const float *dX, const float *dY, const float *dM, const int *didx, int n,
+                       float inv_count) {
+  cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NetGrad<kRows>));
+  const int blocks = std::min((n - 1) / kRows + 1, m->sms);
+  mlp_grad_kernel<<<blocks, kThreads, sizeof(NetGrad<kRows>)>>>(m->P, dX, dY, dM, didx, n, m->norm, inv_count, m->G, m->loss);
+  return check_cuda(cudaGetLastError(), "mlp gradient kernel");
+}
+
+// The launch of the training cluster (`attr`: room for its attribute).
+static cudaLaunchConfig_t train_launch(cudaLaunchAttribute *attr) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(kCluster);
+  lc.blockDim = dim3(kThreads);
+  lc.dynamicSmemBytes = sizeof(NetGrad<kTrainRows>);
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = kCluster;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  return lc;
+}
+
+// Whether the device runs a cluster of this size (16 CTAs are more than every
+// device promises); asked once per network.
+static bool cluster_fits(nvshmemx_mlp *m) {
+  if (m->cluster < 0) {
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t lc = train_launch(&attr);
+    int clusters = 0;
+    const bool ok =
+        cudaFuncSetAttribute(train_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)lc.dynamicSmemBytes) == cudaSuccess &&
+        cudaFuncSetAttribute(train_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, train_cluster_kernel, &lc) == cudaSuccess && clusters > 0;
+    if (!ok) (void)cudaGetLastError();
+    m->cluster = ok ? 1 : 0;
+  }
+  return m->cluster == 1;
+}
+
+static int launch_train(nvshmemx_mlp *m, const float *dX, const float *dY, const float *dM, const int *didx,
+                        const TrainTile *dtiles, int ntiles, float lr, float *dlosses) {
+  cudaLaunchAttribute attr;
+  cudaLaunchConfig_t lc = train_launch(&attr);
+  return check_cuda(cudaLaunchKernelEx(&lc, train_cluster_kernel, m->P, m->Am, m->Av, dX, dY, dM, didx, dtiles, ntiles,
+                                       (const float *)m->norm, lr, dlosses),
+                    "mlp training kernel");
 }
 
 extern "C" {
@@ -253,18 +680,30 @@ int nvshmemx_mlp_num_params(void) { return NPARAM; }
 int nvshmemx_mlp_create(unsigned long long seed, nvshmemx_mlp **out) {
   if (!out) return fail(NVSHMEMX_ERR_INVALID, "mlp_create: null out");
   nvshmemx_mlp *m = new nvshmemx_mlp();
+  const size_t np = kParBytes, nn = kNormBytes;
   int rc;
-  if ((rc = check_cuda(cudaMalloc(&m->P, NPARAM * 4), "cudaMalloc(mlp)")) ||
-      (rc = check_cuda(cudaMalloc(&m->G, NPARAM * 4), "cudaMalloc(mlp)")) ||
-      (rc = check_cuda(cudaMalloc(&m->Am, NPARAM * 4), "cudaMalloc(mlp)")) ||
-      (rc = check_cuda(cudaMalloc(&m->Av, NPARAM * 4), "cudaMalloc(mlp)")) ||
-      (rc = check_cuda(cudaMalloc(&m->norm, 2 * NI * 4), "cudaMalloc(mlp)")) ||
-      (rc = check_cuda(cudaMalloc(&m->loss, 16), "cudaMalloc(mlp)"))) {
+  if ((rc = check_cuda(cudaGetDevice(&m->dev), "cudaGetDevice")) ||
+      (rc = check_cuda(cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->dev),
+                       "cudaDeviceGetAttribute"))) {
     nvshmemx_mlp_destroy(m);
     return rc;
   }
+  m->slot = take_slot(m->dev, &m->block);
+  if (m->slot >= 0) {
+    m->work = m->block + kNetBytes;
+    m->work_bytes = kSlotWork;
+  } else if ((rc = check_cuda(cudaMalloc(&m->block, kNetBytes), "cudaMalloc(mlp)"))) {
+    nvshmemx_mlp_destroy(m);
+    return rc;
+  }
+  m->P = (float *)m->block;
+  m->norm = (float *)(m->block + np);
+  m->Am = (float *)(m->block + np + nn);
+  m->Av = (float *)(m->block + 2 * np + nn);
+  m->G = (float *)(m->block + 3 * np + nn);
+  m->loss = (float *)(m->block + 4 * np + nn);
   // He initialisation: N(0, 2 / fan_in) by Box-Muller on a splitmix64 stream
-  std::vector<float> p(NPARAM, 0.f);
+  std::vector<float> p((np + nn) / 4, 0.f);  // weights, then the normalisation
   unsigned long long ctr = seed;
   auto normal = [&]() {
     const double u1 = ((mix64(ctr++) >> 11) + 1.0) * (1.0 / 9007199254740993.0);
@@ -279,20 +718,25 @@ int nvshmemx_mlp_create(unsigned long long seed, nvshmemx_mlp **out) {
   fill(OFF_W2, NH * NH, NH);
   fill(OFF_W3, NH * NH, NH);
   fill(OFF_W4, NO * NH, NH);
-  cudaMemcpy(m->P, p.data(), NPARAM * 4, cudaMemcpyHostToDevice);
-  cudaMemset(m->Am, 0, NPARAM * 4);
-  cudaMemset(m->Av, 0, NPARAM * 4);
-  const float norm[2 * NI] = {0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 1, 1};
-  cudaMemcpy(m->norm, norm, sizeof norm, cudaMemcpyHostToDevice);
+  for (int i = 0; i < NI; ++i) p[np / 4 + NI + i] = 1.f;
+  if ((rc = upload(m->block, p.data(), np + nn)) ||
+      (rc = check_cuda(cudaMemset(m->Am, 0, 3 * np + 256), "cudaMemset(mlp)"))) {
+    nvshmemx_mlp_destroy(m);
+    return rc;
+  }
   *out = m;
   return check_cuda(cudaDeviceSynchronize(), "mlp_create");
 }
 
 int nvshmemx_mlp_destroy(nvshmemx_mlp *m) {
   if (!m) return 0;
-  float *bufs[] = {m->P, m->G, m->Am, m->Av, m->norm, m->loss};
-  for (float *b : bufs)
-    if (b) cudaFree(b);
+  if (m->work_own) cudaFree(m->work);
+  if (m->slot >= 0) {
+    cudaStreamSynchronize(0);  // nothing of this network runs any more (a free would wait too)
+    give_slot(m->dev, m->slot);
+  } else if (m->block) {
+    cudaFree(m->block);
+  }
   delete m;
   return 0;
 }
@@ -320,11 +764,12 @@ int nvshmemx_mlp_set_normalization(nvshmemx_mlp *m, const float *mean, const flo
 int nvshmemx_mlp_forward(nvshmemx_mlp *m, const float *X, int n, float *Y) {
   if (!m || n < 0 || (n && (!X || !Y))) return fail(NVSHMEMX_ERR_INVALID, "mlp_forward");
   if (n == 0) return 0;
-  DevArr dX, dY;
+  Work w(m);
+  const size_t xb = pad256((size_t)n * NI * 4), yb = (size_t)n * NO * 4;
   int rc;
-  if ((rc = upload(dX, X, (size_t)n * NI * 4)) || (rc = upload(dY, nullptr, (size_t)n * NO * 4))) return rc;
-  if ((rc = mlp_launch(m, false, (float *)dX.p, nullptr, nullptr, nullptr, n, 0.f, (float *)dY.p))) return rc;
-  return check_cuda(cudaMemcpy(Y, dY.p, (size_t)n * NO * 4, cudaMemcpyDeviceToHost), "mlp_forward");
+  if ((rc = w.get(m, xb + yb)) || (rc = upload(w.p, X, (size_t)n * NI * 4))) return rc;
+  if ((rc = launch_forward(m, (float *)w.p, n, (float *)(w.p + xb)))) return rc;
+  return check_cuda(cudaMemcpy(Y, w.p + xb, yb, cudaMemcpyDeviceToHost), "mlp_forward");
 }
 
 int nvshmemx_mlp_loss_grad(nvshmemx_mlp *m, const float *X, const float *Y, const float *M, int n, float *loss,
@@ -333,15 +778,16 @@ int nvshmemx_mlp_loss_grad(nvshmemx_mlp *m, const float *X, const float *Y, cons
   double cnt = 0;
   for (size_t i = 0; i < (size_t)n * NO; ++i) cnt += M[i];
   if (cnt <= 0) return fail(NVSHMEMX_ERR_INVALID, "mlp_loss_grad: empty mask");
-  DevArr dX, dY, dM;
+  Work w(m);
+  const size_t xb = pad256((size_t)n * NI * 4), yb = pad256((size_t)n * NO * 4);
   int rc;
-  if ((rc = upload(dX, X, (size_t)n * NI * 4)) || (rc = upload(dY, Y, (size_t)n * NO * 4)) ||
-      (rc = upload(dM, M, (size_t)n * NO * 4)))
+  if ((rc = w.get(m, xb + 2 * yb)) || (rc = upload(w.p, X, (size_t)n * NI * 4)) ||
+      (rc = upload(w.p + xb, Y, (size_t)n * NO * 4)) || (rc = upload(w.p + xb + yb, M, (size_t)n * NO * 4)))
     return rc;
   cudaMemset(m->G, 0, NPARAM * 4);
   cudaMemset(m->loss, 0, 4);
-  if ((rc = mlp_launch(m, true, (float *)dX.p, (float *)dY.p, (float *)dM.p, nullptr, n, (float)(1.0 / cnt),
-                       nullptr)))
+  if ((rc = launch_grad(m, (float *)w.p, (float *)(w.p + xb), (float *)(w.p + xb + yb), nullptr, n,
+                        (float)(1.0 / cnt))))
     return rc;
   if (loss && (rc = check_cuda(cudaMemcpy(loss, m->loss, 4, cudaMemcpyDeviceToHost), "mlp loss"))) return rc;
   if (grad) return check_cuda(cudaMemcpy(grad, m->G, NPARAM * 4, cudaMemcpyDeviceToHost), "mlp grad");
@@ -351,41 +797,86 @@ int nvshmemx_mlp_loss_grad(nvshmemx_mlp *m, const float *X, const float *Y, cons
 int nvshmemx_mlp_train(nvshmemx_mlp *m, const float *X, const float *Y, const float *M, int n, int epochs, int batch,
                        float lr, unsigned long long seed, float *curve) {
   if (!m || n < 1 || epochs < 1 || batch < 1 || !X || !Y || !M) return fail(NVSHMEMX_ERR_INVALID, "mlp_train");
-  DevArr dX, dY, dM, dI;
-  int rc;
-  if ((rc = upload(dX, X, (size_t)n * NI * 4)) || (rc = upload(dY, Y, (size_t)n * NO * 4)) ||
-      (rc = upload(dM, M, (size_t)n * NO * 4)) || (rc = upload(dI, nullptr, (size_t)n * 4)))
-    return rc;
-  std::vector<int> perm(n);
   std::vector<double> rowm(n, 0.0);
   for (int i = 0; i < n; ++i)
     for (int k = 0; k < NO; ++k) rowm[i] += M[(size_t)i * NO + k];
-  for (int e = 0; e < epochs; ++e) {
-    for (int i = 0; i < n; ++i) perm[i] = i;
-    unsigned long long st = seed * 0x100000001b3ull + (unsigned long long)e;
-    for (int i = n - 1; i > 0; --i) std::swap(perm[i], perm[mix64(st++) % (unsigned long long)(i + 1)]);
-    if ((rc = check_cuda(cudaMemcpy(dI.p, perm.data(), (size_t)n * 4, cudaMemcpyHostToDevice), "mlp idx"))) return rc;
-    cudaMemset(m->loss, 0, 4);
-    int nb = 0;
-    for (int b0 = 0; b0 < n; b0 += batch, ++nb) {
-      const int cnt = std::min(batch, n - b0);
-      double c = 0;
-      for (int i = b0; i < b0 + cnt; ++i) c += rowm[perm[i]];
-      if (c <= 0) continue;
-      cudaMemsetAsync(m->G, 0, NPARAM * 4);
-      if ((rc = mlp_launch(m, true, (float *)dX.p, (float *)dY.p, (float *)dM.p, (int *)dI.p + b0, cnt,
-                           (float)(1.0 / c), nullptr)))
-        return rc;
-      ++m->step;
-      const float c1 = 1.f - powf(0.9f, (float)m->step), c2 = 1.f - powf(0.999f, (float)m->step);
-      adam_kernel<<<(NPARAM + 255) / 256, 256>>>(m->P, m->G, m->Am, m->Av, NPARAM, lr, c1, c2);
-    }
-    if (curve) {
-      float l = 0;
-      if ((rc = check_cuda(cudaMemcpy(&l, m->loss, 4, cudaMemcpyDeviceToHost), "mlp loss"))) return rc;
-      curve[e] = nb ? l / nb : 0.f;
-    }
+  const bool one_cluster = batch <= kClusterBatch && cluster_fits(m);
+  const int nb = (n - 1) / batch + 1;  // batches of an epoch
+  // epochs to a launch: at most 4 MiB of row numbers
+  const int per = one_cluster ? (int)std::min<size_t>((size_t)epochs, std::max<size_t>(1, (1u << 20) / (size_t)n)) : 1;
+  const size_t tiles_epoch = (size_t)nb * ((std::min(n, batch) - 1) / kTileRows + 1);
+  // one block: features, targets, masks, row numbers, tiles, losses
+  const size_t xb = pad256((size_t)n * NI * 4), yb = pad256((size_t)n * NO * 4), ib = pad256((size_t)per * n * 4),
+               tb = one_cluster ? pad256(per * tiles_epoch * sizeof(TrainTile)) : 0, lb = pad256((size_t)epochs * 4);
+  Work w(m);
+  int rc;
+  if ((rc = w.get(m, xb + 2 * yb + ib + tb + lb))) return rc;
+  float *dX = (float *)w.p, *dY = (float *)(w.p + xb), *dM = (float *)(w.p + xb + yb);
+  int *dI = (int *)(w.p + xb + 2 * yb);
+  TrainTile *dT = (TrainTile *)(w.p + xb + 2 * yb + ib);
+  float *dL = (float *)(w.p + xb + 2 * yb + ib + tb);
+  // A table of the usual size goes up in one copy with the first launch's
+  // rows and tiles; a large one array by array.
+  const bool together = one_cluster && n <= 8192;
+  std::vector<char> up((together ? xb + 2 * yb : 0) + ib + tb);
+  if (together) {
+    memcpy(up.data(), X, (size_t)n * NI * 4);
+    memcpy(up.data() + xb, Y, (size_t)n * NO * 4);
+    memcpy(up.data() + xb + yb, M, (size_t)n * NO * 4);
+  } else if ((rc = upload(dX, X, (size_t)n * NI * 4)) || (rc = upload(dY, Y, (size_t)n * NO * 4)) ||
+             (rc = upload(dM, M, (size_t)n * NO * 4))) {
+    return rc;
   }
+  char *const hrows = up.data() + (together ? xb + 2 * yb : 0);
+  if ((rc = check_cuda(cudaMemsetAsync(dL, 0, lb), "cudaMemsetAsync(losses)"))) return rc;
+  for (int e0 = 0; e0 < epochs; e0 += per) {
+    const int e1 = std::min(epochs, e0 + per);
+    int *perm = (int *)hrows;
+    TrainTile *tiles = (TrainTile *)(hrows + ib);
+    size_t nt = 0;
+    for (int e = e0; e < e1; ++e, perm += n) {
+      for (int i = 0; i < n; ++i) perm[i] = i;
+      unsigned long long st = seed * 0x100000001b3ull + (unsigned long long)e;
+      for (int i = n - 1; i > 0; --i) std::swap(perm[i], perm[mix64(st++) % (unsigned long long)(i + 1)]);
+      if (!one_cluster) {
+        if ((rc = upload(dI, perm, (size_t)n * 4))) return rc;
+        cudaMemsetAsync(m->loss, 0, 4);
+      }
+      for (int b0 = 0; b0 < n; b0 += batch) {
+        const int cnt = std::min(batch, n - b0);
+        double c = 0;
+        for (int i = b0; i < b0 + cnt; ++i) c += rowm[perm[i]];
+        if (c <= 0) continue;
+        ++m->step;
+        const float c1 = 1.f - powf(0.9f, (float)m->step), c2 = 1.f - powf(0.999f, (float)m->step);
+        if (one_cluster) {
+          for (int k = 0; k < cnt; k += kTileRows) {
+            const bool last = cnt - k <= kTileRows;
+            tiles[nt++] = TrainTile{(e - e0) * n + b0 + k, std::min(cnt - k, kTileRows), (float)(1.0 / c), c1, c2,
+                                    (k == 0 ? kFirst : 0) | (last ? kLast : 0), e, 0};
+          }
+        } else {
+          cudaMemsetAsync(m->G, 0, NPARAM * 4);
+          if ((rc = launch_grad(m, dX, dY, dM, dI + b0, cnt, (float)(1.0 / c)))) return rc;
+          adam_kernel<<<(NPARAM + 255) / 256, 256>>>(m->P, m->G, m->Am, m->Av, NPARAM, lr, c1, c2);
+        }
+      }
+      if (!one_cluster && curve &&
+          (rc = check_cuda(cudaMemcpy(&curve[e], m->loss, 4, cudaMemcpyDeviceToHost), "mlp loss")))
+        return rc;
+    }
+    if (!one_cluster) continue;
+    const bool first_up = together && e0 == 0;
+    if ((rc = first_up ? upload(w.p, up.data(), xb + 2 * yb + ib + nt * sizeof(TrainTile))
+                       : upload(dI, hrows, ib + nt * sizeof(TrainTile))))
+      return rc;
+    if (nt && (rc = launch_train(m, dX, dY, dM, dI, dT, (int)nt, lr, dL))) return rc;
+  }
+  if (one_cluster && curve &&
+      (rc = check_cuda(cudaMemcpy(curve, dL, (size_t)epochs * 4, cudaMemcpyDeviceToHost), "mlp losses")))
+    return rc;
+  if (curve)
+    for (int e = 0; e < epochs; ++e) curve[e] /= (float)nb;
   return check_cuda(cudaDeviceSynchronize(), "mlp_train");
 }
 
