@@ -106,6 +106,75 @@ __device__ __forceinline__ nvshmemx_request expand_compact(const uint4 q) {
   return r;
 }
 
+// A request as a work item and the number of chunks it is cut into (0 bytes:
+// none).  Returns 0 or the error that planning reports.
+__device__ __forceinline__ int plan_one(const Cfg &c, const nvshmemx_request &r, unsigned chunk, WorkItem &w,
+                                        unsigned &cnt) {
+  cnt = 0;
+  w.dst = w.src = 0;
+  w.len = 0;
+  w.kind = kCopy;
+  w.value = 0;
+  w.pad = 0;
+  const unsigned width = r.dtype == NVSHMEMX_DT_DOUBLE ? 8u : 4u;
+  const bool pe_ok = r.src_pe < c.npes && r.dst_pe < c.npes && r.dtype <= NVSHMEMX_DT_DOUBLE;
+  const unsigned long long dst = (unsigned long long)c.arena + ((unsigned long long)r.dst_pe << c.log2_stride) + r.dst_off;
+  const unsigned long long src = (unsigned long long)c.arena + ((unsigned long long)r.src_pe << c.log2_stride) + r.src_off;
+  switch (r.op) {
+    case NVSHMEMX_REQ_PUT:
+    case NVSHMEMX_REQ_GET:
+    case NVSHMEMX_REQ_G: {
+      const unsigned long long bytes = r.op == NVSHMEMX_REQ_G ? width : r.bytes;
+      if (!pe_ok || !range_in_slice(c, r.src_off, bytes) || !range_in_slice(c, r.dst_off, bytes))
+        return NVSHMEMX_ERR_BOUNDS;
+      w.dst = dst;
+      w.src = src;
+      w.len = (unsigned)bytes;
+      cnt = bytes ? (unsigned)((bytes + chunk - 1) / chunk) : 0u;
+      return 0;
+    }
+    case NVSHMEMX_REQ_SIGNAL:
+    case NVSHMEMX_REQ_P: {
+      const unsigned bytes = r.op == NVSHMEMX_REQ_SIGNAL ? 4u : width;
+      if (!pe_ok || !range_in_slice(c, r.dst_off, bytes) || (r.dst_off & (bytes - 1))) return NVSHMEMX_ERR_BOUNDS;
+      w.dst = dst;
+      w.src = r.src_off;
+      w.len = bytes;
+      w.kind = r.op == NVSHMEMX_REQ_SIGNAL ? kSignal : kStore;
+      w.value = r.value;
+      cnt = 1;
+      return 0;
+    }
+    default:
+      return NVSHMEMX_ERR_INVALID;
+  }
+}
+
+// Chunk k of a planned request, `chunk` bytes each.
+__device__ __forceinline__ WorkItem chunk_of(const WorkItem &w, unsigned long long k, unsigned chunk) {
+  WorkItem p = w;
+  if (w.kind == kCopy) {
+    const unsigned long long off = k * chunk;
+    p.dst += off;
+    p.src += off;
+    p.len = (unsigned)((w.len - off) < chunk ? (w.len - off) : chunk);
+  }
+  return p;
+}
+
+__device__ __forceinline__ nvshmemx_request load_request(const void *reqs, int i, bool compact) {
+  if (compact) return expand_compact(reinterpret_cast<const uint4 *>(reqs)[i]);
+  return reinterpret_cast<const nvshmemx_request *>(reqs)[i];
+}
+
+__device__ __forceinline__ void store_request(nvshmemx_request *p, const nvshmemx_request &r) {
+  uint4 lo, hi;
+  memcpy(&lo, &r, 16);
+  memcpy(&hi, reinterpret_cast<const char *>(&r) + 16, 16);
+  reinterpret_cast<uint4 *>(p)[0] = lo;
+  reinterpret_cast<uint4 *>(p)[1] = hi;
+}
+
 // A batch is planned as one piece, or (pipelined submit) as consecutive
 // pieces planned in order on one stream: piece k appends its items after
 // those of piece k-1 (`prev`) and reports errors, with request indices offset
@@ -132,60 +201,11 @@ __global__ void __launch_bounds__(kPlanThreads) batch_plan_kernel(Cfg c, const v
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   unsigned cnt = 0;
   WorkItem w;
-  w.dst = w.src = 0;
-  w.len = 0;
-  w.kind = kCopy;
-  w.value = 0;
-  w.pad = 0;
   if (i < n) {
-    nvshmemx_request r;
-    if (COMPACT) {
-      r = expand_compact(reinterpret_cast<const uint4 *>(reqs_in)[i]);
-      uint4 lo, hi;
-      memcpy(&lo, &r, 16);
-      memcpy(&hi, reinterpret_cast<const char *>(&r) + 16, 16);
-      reinterpret_cast<uint4 *>(keep + i)[0] = lo;
-      reinterpret_cast<uint4 *>(keep + i)[1] = hi;
-    } else {
-      r = reinterpret_cast<const nvshmemx_request *>(reqs_in)[i];
-    }
-    const unsigned width = r.dtype == NVSHMEMX_DT_DOUBLE ? 8u : 4u;
-    const bool pe_ok = r.src_pe < c.npes && r.dst_pe < c.npes && r.dtype <= NVSHMEMX_DT_DOUBLE;
-    const unsigned long long dst = (unsigned long long)c.arena + ((unsigned long long)r.dst_pe << c.log2_stride) + r.dst_off;
-    const unsigned long long src = (unsigned long long)c.arena + ((unsigned long long)r.src_pe << c.log2_stride) + r.src_off;
-    switch (r.op) {
-      case NVSHMEMX_REQ_PUT:
-      case NVSHMEMX_REQ_GET:
-      case NVSHMEMX_REQ_G: {
-        const unsigned long long bytes = r.op == NVSHMEMX_REQ_G ? width : r.bytes;
-        if (!pe_ok || !range_in_slice(c, r.src_off, bytes) || !range_in_slice(c, r.dst_off, bytes)) {
-          set_status(sctl, NVSHMEMX_ERR_BOUNDS, req_base + i);
-          break;
-        }
-        w.dst = dst;
-        w.src = src;
-        w.len = (unsigned)bytes;
-        cnt = bytes ? (unsigned)((bytes + chunk - 1) / chunk) : 0u;
-        break;
-      }
-      case NVSHMEMX_REQ_SIGNAL:
-      case NVSHMEMX_REQ_P: {
-        const unsigned bytes = r.op == NVSHMEMX_REQ_SIGNAL ? 4u : width;
-        if (!pe_ok || !range_in_slice(c, r.dst_off, bytes) || (r.dst_off & (bytes - 1))) {
-          set_status(sctl, NVSHMEMX_ERR_BOUNDS, req_base + i);
-          break;
-        }
-        w.dst = dst;
-        w.src = r.src_off;
-        w.len = bytes;
-        w.kind = r.op == NVSHMEMX_REQ_SIGNAL ? kSignal : kStore;
-        w.value = r.value;
-        cnt = 1;
-        break;
-      }
-      default:
-        set_status(sctl, NVSHMEMX_ERR_INVALID, req_base + i);
-    }
+    const nvshmemx_request r = load_request(reqs_in, i, COMPACT);
+    if (COMPACT) store_request(keep + i, r);
+    const int err = plan_one(c, r, chunk, w, cnt);
+    if (err) set_status(sctl, err, req_base + i);
   }
   // CTA-wide exclusive scan of cnt
   unsigned incl = cnt;
@@ -210,18 +230,7 @@ __global__ void __launch_bounds__(kPlanThreads) batch_plan_kernel(Cfg c, const v
   if (cnt == 0) return;
   const unsigned long long first = ibase + block_base + warp_sums[warp] + (incl - cnt);
   if (first + cnt > cap) return;
-  if (cnt == 1) {
-    items[first] = w;
-    return;
-  }
-  for (unsigned k = 0; k < cnt; ++k) {
-    WorkItem p = w;
-    const unsigned long long off = (unsigned long long)k * chunk;
-    p.dst += off;
-    p.src += off;
-    p.len = (unsigned)((w.len - off) < chunk ? (w.len - off) : chunk);
-    items[first + k] = p;
-  }
+  for (unsigned k = 0; k < cnt; ++k) items[first + k] = chunk_of(w, k, chunk);
 }
 
 // ------------------------------------------------------------------- exec
@@ -432,6 +441,173 @@ __global__ void __launch_bounds__(256, 3) batch_exec_tma_kernel(const WorkItem *
   }
 }
 
+// ------------------------------------------------ small batches: one launch
+// Below kSmallRequests requests, planning is done by every CTA for itself: it
+// reads all requests (at most 128 KB, from L2 or, for a few, from the kernel's
+// parameters), checks them, and builds the running count of pieces in its own
+// shared memory.  No CTA waits for another and nothing has to be zeroed, so
+// the memset, the plan kernel and the exec kernel become one launch; an
+// invalid request is seen by every CTA, and none copies anything.  Pieces are
+// a power of two of bytes, at most the configured chunk and about two for
+// each warp of the grid, so a batch of few requests still spreads over every
+// SM (with 16 KiB chunks a 64-request batch keeps some 80 of 1184 warps
+// busy).  CTA b takes pieces b, b + gridDim.x, ..., its warps the next one
+// each.  Measured per call from pinned memory: 64 requests 49 -> 29 us, 1000
+// requests 51 -> 36 us, 2999 requests 56 -> 49 us (98 -> 53 us with sources off
+// by 4 to 12 bytes).  From some 5000 requests on, reading every request in
+// every CTA costs more than a plan kernel (6000: 65 against 62 us).
+constexpr int kSmallRequests = 4096;
+constexpr int kParamWords = 240;  // 16-byte words of requests that fit the kernel's parameters
+
+template <int NP>
+struct ReqParams {
+  uint4 q[NP];
+};
+
+struct SmallShared {  // behind the rings
+  unsigned long long bytes, chunks;
+  unsigned err;     // smallest (request << 8 | code), ~0 when all are valid
+  unsigned next;    // pieces claimed by this CTA
+  unsigned total;   // pieces of the batch
+  unsigned warp[8];
+  unsigned pre[1];  // pieces before entry s; entry (i % T) * stride + i / T is request i
+                    // (an odd stride: a thread's entries are consecutive)
+};
+
+static size_t small_smem_bytes(const nvshmemx_batch_config &k, int n) {
+  const size_t entries = (size_t)k.threads * (((n + k.threads - 1) / k.threads) | 1);
+  return (size_t)(k.threads / 32) * (256 + (size_t)k.tma_stages * (size_t)k.tma_stage_bytes) + sizeof(SmallShared) +
+         entries * sizeof(unsigned);
+}
+
+template <int S, int NP>
+__global__ void __launch_bounds__(256, 3)
+    batch_small_kernel(const __grid_constant__ ReqParams<NP> par, Cfg c, const void *reqs, int n, int compact,
+                       unsigned chunk, unsigned long long cap, nvshmemx_request *keep, BatchCtl *ctl, int *host,
+                       unsigned SB, unsigned min_bulk) {
+  extern __shared__ __align__(128) char smem[];
+  const unsigned t = threadIdx.x, T = blockDim.x, lane = t & 31u, warp = t >> 5;
+  WarpTma<S> ring;
+  ring.init(smem, SB, min_bulk, c.wait_timeout_ns, lane);
+  SmallShared &sh = *reinterpret_cast<SmallShared *>(smem + (size_t)(T >> 5) * (256 + (size_t)S * SB));
+  const void *src = NP > 1 ? static_cast<const void *>(par.q) : reqs;
+  const unsigned per = (((unsigned)n + T - 1) / T) | 1u;  // odd: the threads' entries fall into different banks
+  if (t == 0) {
+    sh.bytes = sh.chunks = 0;
+    sh.err = ~0u;
+    sh.next = 0;
+  }
+  __syncthreads();
+  // every request: its size in 16-byte units (scalar stores: the top bit)
+  unsigned long long bytes = 0, chunks = 0;
+  unsigned err = ~0u;
+  for (unsigned k = 0; k < per; ++k) {
+    const unsigned i = t + k * T;
+    unsigned units = 0;
+    if (i < (unsigned)n) {
+      const nvshmemx_request r = load_request(src, (int)i, compact != 0);
+      if (keep && blockIdx.x == 0) store_request(keep + i, r);
+      WorkItem w;
+      unsigned cnt;
+      const int e = plan_one(c, r, chunk, w, cnt);
+      if (e) {
+        const unsigned code = (i << 8) | (unsigned)e;
+        err = code < err ? code : err;
+      } else {
+        chunks += cnt;
+        if (w.kind == kCopy) {
+          bytes += w.len;
+          units = (unsigned)((w.len + 15ull) >> 4);
+        } else {
+          units = 1u << 31;
+        }
+      }
+    }
+    sh.pre[t * per + k] = units;
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
+    chunks += __shfl_xor_sync(0xffffffffu, chunks, o);
+    const unsigned e = __shfl_xor_sync(0xffffffffu, err, o);
+    err = e < err ? e : err;
+  }
+  if (lane == 0) {
+    atomicAdd(&sh.bytes, bytes);
+    atomicAdd(&sh.chunks, chunks);
+    atomicMin(&sh.err, err);
+  }
+  __syncthreads();
+  if (blockIdx.x == 0 && t == 0) {
+    ctl->total_chunks = sh.chunks;
+    ctl->item_base = 0;
+    if (sh.err != ~0u) {
+      host[1] = (int)(sh.err >> 8);
+      host[0] = (int)(sh.err & 255u);
+    } else if (sh.chunks > cap) {
+      host[1] = -1;
+      host[0] = NVSHMEMX_ERR_NOMEM;
+    }
+  }
+  const bool run = sh.err == ~0u && sh.chunks <= cap;
+  // bytes of a piece, as a power of two: about two pieces for each warp of
+  // the grid, from 1 KiB to the chunk, and fewer than 2^31 pieces in all
+  const unsigned max_lg = 31 - __clz(chunk);
+  const unsigned long long want = sh.bytes / (2ull * gridDim.x * (T >> 5));
+  unsigned lg = want > 1024 ? 64 - __clzll(want - 1) : 10;
+  if (lg > max_lg) lg = max_lg;
+  if (sh.bytes >> 30) {
+    const unsigned least = 64 - __clzll(sh.bytes >> 30);
+    if (lg < least) lg = least;
+  }
+  // running count of pieces: within the thread, over the warp, over the CTA
+  unsigned sum = 0;
+  for (unsigned k = 0; k < per; ++k) {
+    const unsigned u = sh.pre[t * per + k];
+    sh.pre[t * per + k] = sum;
+    sum += (u >> 31) ? 1u : (unsigned)((u + (1ull << (lg - 4)) - 1) >> (lg - 4));
+  }
+  unsigned incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= (unsigned)o) incl += v;
+  }
+  if (lane == 31) sh.warp[warp] = incl;
+  __syncthreads();
+  unsigned before = incl - sum;
+  for (unsigned k = 0; k < warp; ++k) before += sh.warp[k];
+  for (unsigned k = 0; k < per; ++k) sh.pre[t * per + k] += before;
+  if (t == T - 1) sh.total = before + sum;
+  __syncthreads();
+  const unsigned total = run ? sh.total : 0u, entries = per * T;
+  for (;;) {
+    unsigned l = 0;
+    if (lane == 0) l = atomicAdd(&sh.next, 1u);
+    l = __shfl_sync(0xffffffffu, l, 0);
+    const unsigned long long g = blockIdx.x + (unsigned long long)l * gridDim.x;
+    if (g >= total) break;
+    // the last entry with at most g pieces before it: 32 probes at a time
+    unsigned lo = 0, size = entries;
+    while (size > 1) {
+      const unsigned step = (size + 31) / 32, at = lane * step;
+      const bool le = at < size && sh.pre[lo + at] <= g;
+      const unsigned k = __popc(__ballot_sync(0xffffffffu, le)) - 1;
+      lo += k * step;
+      size = size - k * step < step ? size - k * step : step;
+    }
+    const nvshmemx_request r = load_request(src, (int)(lo / per + (lo % per) * T), compact != 0);
+    WorkItem w;
+    unsigned cnt;
+    plan_one(c, r, chunk, w, cnt);
+    ring.run(chunk_of(w, g - sh.pre[lo], 1u << lg), lane);
+  }
+  if (!ring.drain(lane) && lane == 0) {
+    host[1] = -2;
+    host[0] = NVSHMEMX_ERR_TIMEOUT;
+  }
+}
+
 // ------------------------------------------------ streaming: one launch
 // Planning and execution in one persistent cooperative launch.  The first
 // `planners` warps of every CTA claim groups of 32 requests in request order
@@ -460,53 +636,6 @@ struct StreamCtl {                 // the first 32 bytes match BatchCtl
 };
 static_assert(sizeof(StreamCtl) == 64, "StreamCtl is one 64-byte block");
 
-__device__ __forceinline__ void plan_one(const Cfg &c, const nvshmemx_request &r, int i, unsigned chunk,
-                                         BatchCtl *ctl, WorkItem &w, unsigned &cnt) {
-  cnt = 0;
-  w.dst = w.src = 0;
-  w.len = 0;
-  w.kind = kCopy;
-  w.value = 0;
-  w.pad = 0;
-  const unsigned width = r.dtype == NVSHMEMX_DT_DOUBLE ? 8u : 4u;
-  const bool pe_ok = r.src_pe < c.npes && r.dst_pe < c.npes && r.dtype <= NVSHMEMX_DT_DOUBLE;
-  const unsigned long long dst = (unsigned long long)c.arena + ((unsigned long long)r.dst_pe << c.log2_stride) + r.dst_off;
-  const unsigned long long src = (unsigned long long)c.arena + ((unsigned long long)r.src_pe << c.log2_stride) + r.src_off;
-  switch (r.op) {
-    case NVSHMEMX_REQ_PUT:
-    case NVSHMEMX_REQ_GET:
-    case NVSHMEMX_REQ_G: {
-      const unsigned long long bytes = r.op == NVSHMEMX_REQ_G ? width : r.bytes;
-      if (!pe_ok || !range_in_slice(c, r.src_off, bytes) || !range_in_slice(c, r.dst_off, bytes)) {
-        set_status(ctl, NVSHMEMX_ERR_BOUNDS, i);
-        return;
-      }
-      w.dst = dst;
-      w.src = src;
-      w.len = (unsigned)bytes;
-      cnt = bytes ? (unsigned)((bytes + chunk - 1) / chunk) : 0u;
-      return;
-    }
-    case NVSHMEMX_REQ_SIGNAL:
-    case NVSHMEMX_REQ_P: {
-      const unsigned bytes = r.op == NVSHMEMX_REQ_SIGNAL ? 4u : width;
-      if (!pe_ok || !range_in_slice(c, r.dst_off, bytes) || (r.dst_off & (bytes - 1))) {
-        set_status(ctl, NVSHMEMX_ERR_BOUNDS, i);
-        return;
-      }
-      w.dst = dst;
-      w.src = r.src_off;
-      w.len = bytes;
-      w.kind = r.op == NVSHMEMX_REQ_SIGNAL ? kSignal : kStore;
-      w.value = r.value;
-      cnt = 1;
-      return;
-    }
-    default:
-      set_status(ctl, NVSHMEMX_ERR_INVALID, i);
-  }
-}
-
 // The item's payload (its first 28 bytes), written with plain stores; the
 // generation tag in the last word is stored separately, after a fence.
 __device__ __forceinline__ void write_item_body(WorkItem *p, const WorkItem &w) {
@@ -532,7 +661,7 @@ __device__ __forceinline__ WorkItem read_item(const WorkItem *p) {
   return w;
 }
 
-__device__ __forceinline__ nvshmemx_request load_request(const nvshmemx_request *p) {
+__device__ __forceinline__ nvshmemx_request load_request_cg(const nvshmemx_request *p) {
   const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(p));
   const uint4 b = __ldcg(reinterpret_cast<const uint4 *>(p) + 1);
   nvshmemx_request r;
@@ -596,16 +725,19 @@ __global__ void __launch_bounds__(256) batch_stream_kernel(Cfg c, const nvshmemx
     };
     int g = claim();
     nvshmemx_request r;
-    if (g < ngroups && g * 32 + (int)lane < n) r = load_request(reqs + g * 32 + lane);
+    if (g < ngroups && g * 32 + (int)lane < n) r = load_request_cg(reqs + g * 32 + lane);
     while (g < ngroups) {
       const int i = g * 32 + (int)lane;
       // claim the next group and fetch it while this one is planned
       const int gn = claim();
       nvshmemx_request rn;
-      if (gn < ngroups && gn * 32 + (int)lane < n) rn = load_request(reqs + gn * 32 + lane);
+      if (gn < ngroups && gn * 32 + (int)lane < n) rn = load_request_cg(reqs + gn * 32 + lane);
       WorkItem w;
       unsigned cnt = 0;
-      if (i < n) plan_one(c, r, i, chunk, bctl, w, cnt);
+      if (i < n) {
+        const int err = plan_one(c, r, chunk, w, cnt);
+        if (err) set_status(bctl, err, i);
+      }
       unsigned incl = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -621,14 +753,7 @@ __global__ void __launch_bounds__(256) batch_stream_kernel(Cfg c, const nvshmemx
       base = __shfl_sync(0xffffffffu, base, 31);
       const unsigned long long first = base + incl - cnt;
       const unsigned last = first + cnt <= cap ? cnt : (first < cap ? (unsigned)(cap - first) : 0u);
-      for (unsigned k = 0; k < last; ++k) {
-        WorkItem p = w;
-        const unsigned long long off = (unsigned long long)k * chunk;
-        p.dst += off;
-        p.src += off;
-        if (w.kind == kCopy) p.len = (unsigned)((w.len - off) < chunk ? (w.len - off) : chunk);
-        write_item_body(items + first + k, p);
-      }
+      for (unsigned k = 0; k < last; ++k) write_item_body(items + first + k, chunk_of(w, k, chunk));
       // one fence per group orders every payload before its tag (a release
       // pattern: fence, then strong stores); consumers acquire the tag
       __threadfence();
@@ -803,6 +928,11 @@ struct nvshmemx_batch {
   nvshmemx_batch_config graph_cfg{};
   Cfg graph_arena{};
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr, ev_plan0 = nullptr, ev_exec0 = nullptr, ev_exec1 = nullptr;
+  // the small-batch kernel's grid for the configuration and shared memory it
+  // was last asked for
+  nvshmemx_batch_config small_cfg{};
+  size_t small_smem = 0;
+  int small_ctas = 0;
   bool timed_direct = false;  // ev_plan0/ev_exec0/ev_exec1 hold the last direct execution
   int last_pieces = 1;        // pieces of the last execution (pipelined submit: 2)
 };
@@ -966,6 +1096,86 @@ static int ensure_graph(nvshmemx_batch *b, const nvshmemx_request *src) {
   b->graph_cfg = b->cfg;
   b->graph_arena = c;
   return 0;
+}
+
+// ------------------------------------------------------ small batches (host)
+typedef void (*SmallFn)(ReqParams<1>, Cfg, const void *, int, int, unsigned, unsigned long long, nvshmemx_request *,
+                        BatchCtl *, int *, unsigned, unsigned);
+typedef void (*SmallParFn)(ReqParams<kParamWords>, Cfg, const void *, int, int, unsigned, unsigned long long,
+                           nvshmemx_request *, BatchCtl *, int *, unsigned, unsigned);
+
+static SmallFn pick_small(int stages) {
+  switch (stages) {
+    case 2: return batch_small_kernel<2, 1>;
+    case 3: return batch_small_kernel<3, 1>;
+    default: return batch_small_kernel<4, 1>;
+  }
+}
+static SmallParFn pick_small_par(int stages) {
+  switch (stages) {
+    case 2: return batch_small_kernel<2, kParamWords>;
+    case 3: return batch_small_kernel<3, kParamWords>;
+    default: return batch_small_kernel<4, kParamWords>;
+  }
+}
+
+static const size_t kMaxSmem = 227u << 10;
+
+// Whether n requests run as one launch: a TMA configuration whose rings leave
+// room for the running count (the default's do, up to the limit).
+static bool small_batch(const nvshmemx_batch *b, int n) {
+  const nvshmemx_batch_config &k = b->cfg;
+  return n > 0 && n < kSmallRequests && k.stream == 0 && k.tma_stages > 0 && small_smem_bytes(k, n) <= kMaxSmem;
+}
+
+// Enqueues a small batch on the batch's stream: n requests in device memory at
+// `dev`, or (dev null) at `host`, at most kParamWords * 16 bytes, as kernel
+// parameters.  `keep`: where their full form is stored, or null.
+static int enqueue_small(nvshmemx_batch *b, const void *dev, const void *host, int n, bool compact,
+                         nvshmemx_request *keep) {
+  const Runtime &r = rt();
+  const nvshmemx_batch_config &k = b->cfg;
+  const SmallFn fn = pick_small(k.tma_stages);
+  const SmallParFn pfn = pick_small_par(k.tma_stages);
+  const size_t smem = small_smem_bytes(k, n);
+  (void)cudaGetLastError();
+  if (b->small_ctas == 0 || b->small_smem != smem || memcmp(&b->small_cfg, &k, sizeof k) != 0) {
+    for (const void *f : {(const void *)fn, (const void *)pfn}) {
+      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+      cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    }
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, k.threads, smem);
+    if (per_sm < 1) per_sm = 1;
+    b->small_ctas = r.sm_count * (k.ctas_per_sm > 0 && k.ctas_per_sm < per_sm ? k.ctas_per_sm : per_sm);
+    b->small_smem = smem;
+    b->small_cfg = k;
+  }
+  if (dev) {
+    fn<<<b->small_ctas, k.threads, smem, b->stream>>>(ReqParams<1>{}, r.cfg, dev, n, compact, (unsigned)k.chunk_bytes,
+                                                      b->cap, keep, b->d_ctl, b->h_status_dev,
+                                                      (unsigned)k.tma_stage_bytes, (unsigned)k.tma_min_bytes);
+  } else {
+    ReqParams<kParamWords> par;
+    memcpy(&par, host, (size_t)n * (compact ? sizeof(nvshmemx_request_compact) : sizeof(nvshmemx_request)));
+    pfn<<<b->small_ctas, k.threads, smem, b->stream>>>(par, r.cfg, nullptr, n, compact, (unsigned)k.chunk_bytes,
+                                                       b->cap, keep, b->d_ctl, b->h_status_dev,
+                                                       (unsigned)k.tma_stage_bytes, (unsigned)k.tma_min_bytes);
+  }
+  return check_cuda(cudaGetLastError(), "small batch launch");
+}
+
+// A small submit: n requests at `host`, copied to `dev` unless they fit the
+// kernel's parameters.
+static int submit_small(nvshmemx_batch *b, const void *host, void *dev, size_t elem, bool compact, int n) {
+  int rc;
+  const bool params = (size_t)n * elem <= kParamWords * 16;
+  b->last_pieces = 1;
+  b->h_status[0] = b->h_status[1] = 0;
+  if (!params && (rc = check_cuda(cudaMemcpyAsync(dev, host, (size_t)n * elem, cudaMemcpyHostToDevice, b->stream),
+                                  "cudaMemcpyAsync(requests)")))
+    return rc;
+  return enqueue_small(b, params ? nullptr : dev, host, n, compact, params || compact ? b->d_reqs : nullptr);
 }
 
 // ------------------------------------------------ grouped runs (picker.cu)
@@ -1137,18 +1347,22 @@ int nvshmemx_batch_upload(nvshmemx_batch *b, const nvshmemx_request *reqs, int n
 int nvshmemx_batch_execute(nvshmemx_batch *b, int reps, float *out_ms) {
   if (!b || reps < 1) return fail(NVSHMEMX_ERR_INVALID, "batch_execute: bad arguments");
   int rc;
-  if ((rc = ensure_graph(b, b->d_reqs))) return rc;
+  const bool small = small_batch(b, b->n);
+  if (!small && (rc = ensure_graph(b, b->d_reqs))) return rc;
   b->last_pieces = 1;
+  b->h_status[0] = b->h_status[1] = 0;
   cudaEventRecord(b->ev_start, b->stream);
   for (int i = 0; i < reps; ++i)
-    if ((rc = check_cuda(cudaGraphLaunch(b->gexec, b->stream), "cudaGraphLaunch"))) return rc;
+    if ((rc = small ? enqueue_small(b, b->d_reqs, nullptr, b->n, false, nullptr)
+                    : check_cuda(cudaGraphLaunch(b->gexec, b->stream), "cudaGraphLaunch")))
+      return rc;
   cudaEventRecord(b->ev_stop, b->stream);
   if ((rc = check_cuda(cudaStreamSynchronize(b->stream), "batch_execute"))) return rc;
   float ms = 0;
   cudaEventElapsedTime(&ms, b->ev_start, b->ev_stop);
   if (out_ms) *out_ms = ms;
-  int st[2] = {0, 0};
-  cudaMemcpy(st, &b->d_ctl->status, sizeof st, cudaMemcpyDeviceToHost);
+  int st[2] = {b->h_status[0], b->h_status[1]};
+  if (!small) cudaMemcpy(st, &b->d_ctl->status, sizeof st, cudaMemcpyDeviceToHost);
   if (st[0]) return fail(st[0], "batch_execute: request %d rejected (%s)", st[1], nvshmemx_strerror(st[0]));
   return 0;
 }
@@ -1215,12 +1429,15 @@ int nvshmemx_batch_submit(nvshmemx_batch *b, const nvshmemx_request *reqs, int n
   int rc;
   b->n = n;
   int ends[3];
+  const bool small = small_batch(b, n);
   const int pieces = b->cfg.stream ? 1 : split_pieces(n, ends);
-  if (pieces == 1 && (rc = ensure_graph(b, b->d_reqs))) return rc;
+  if (!small && pieces == 1 && (rc = ensure_graph(b, b->d_reqs))) return rc;
   b->last_pieces = pieces;
   b->timed_direct = false;
   cudaEventRecord(b->ev_start, b->stream);
-  if (pieces > 1) {
+  if (small) {
+    if ((rc = submit_small(b, reqs, b->d_reqs, sizeof(nvshmemx_request), false, n))) return rc;
+  } else if (pieces > 1) {
     if ((rc = submit_pieces(b, reqs, b->d_reqs, sizeof(nvshmemx_request), 0, pieces, ends))) return rc;
   } else {
     if (n && (rc = check_cuda(cudaMemcpyAsync(b->d_reqs, reqs, (size_t)n * sizeof(nvshmemx_request),
@@ -1261,7 +1478,9 @@ int nvshmemx_batch_submit_compact(nvshmemx_batch *b, const nvshmemx_request_comp
   const int pieces = split_pieces(n, ends);
   b->last_pieces = pieces;
   cudaEventRecord(b->ev_start, b->stream);
-  if ((rc = submit_pieces(b, reqs, b->d_reqs_compact, sizeof(nvshmemx_request_compact), kCompact, pieces, ends)))
+  if (small_batch(b, n)) {
+    if ((rc = submit_small(b, reqs, b->d_reqs_compact, sizeof(nvshmemx_request_compact), true, n))) return rc;
+  } else if ((rc = submit_pieces(b, reqs, b->d_reqs_compact, sizeof(nvshmemx_request_compact), kCompact, pieces, ends)))
     return rc;
   cudaEventRecord(b->ev_stop, b->stream);
   if ((rc = check_cuda(cudaStreamSynchronize(b->stream), "batch_submit_compact"))) return rc;

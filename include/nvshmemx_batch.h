@@ -35,7 +35,7 @@ extern "C" {
 
 typedef struct nvshmemx_batch_config {
   int vec_bytes;    /* widest access: 4, 8 or 16                              */
-  int chunk_bytes;  /* work unit: multiple of 256 in [256, 1 MiB]             */
+  int chunk_bytes;  /* largest work unit: multiple of 256 in [256, 1 MiB]     */
   int unroll;       /* accesses in flight per lane: 1, 2, 4 or 8              */
   int threads;      /* threads per CTA: 128, 256, 512 or 1024 (TMA: <= 256)   */
   int ctas_per_sm;  /* resident CTAs per SM (0: as many as fit)               */
@@ -87,7 +87,10 @@ int nvshmemx_batch_execute(nvshmemx_batch *b, int reps, float *out_ms);
 /* End-to-end call: copies n requests from host memory (pinned if it is the
  * batch's host buffer), executes them and reads back the batch status word;
  * *out_status receives the status (0 = every request done), *out_ms the
- * device time of the whole sequence.  With a graph configuration (stream 0)
+ * device time of the whole sequence.  Below 4096 requests a TMA
+ * configuration runs the batch as one launch (no plan kernel, no graph; the
+ * work unit is then at most chunk_bytes), and some hundred requests travel as
+ * the kernel's parameters.  Otherwise, with a graph configuration (stream 0),
  * the copy precedes the plan and exec kernels on the batch's stream; from
  * 8192 requests on, the batch runs as two pieces: a second stream copies
  * and plans the first quarter (in whole 256-request blocks), then the rest,
