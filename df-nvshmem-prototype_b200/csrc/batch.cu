@@ -41,8 +41,16 @@ struct BatchCtl {  // 32 bytes, zeroed before every execution
   unsigned long long item_base;     // index of the piece's first work item
 };
 
-__device__ __forceinline__ void set_status(BatchCtl *ctl, int code, int req) {
-  if (atomicCAS(&ctl->status, 0, code) == 0) ctl->bad_request = req;
+// Records the first error of a control block and, when `host` is given, writes
+// it to the batch's pinned status words, which the host set to 0 before the
+// launch and reads after it has waited for the stream.
+__device__ __forceinline__ void set_status(BatchCtl *ctl, int code, int req, int *host = nullptr) {
+  if (atomicCAS(&ctl->status, 0, code) != 0) return;
+  ctl->bad_request = req;
+  if (host) {
+    host[1] = req;
+    host[0] = code;
+  }
 }
 
 // Programmatic dependent launch: the plan kernel lets the exec kernel start
@@ -191,11 +199,12 @@ __global__ void __launch_bounds__(kPlanThreads) batch_plan_kernel(Cfg c, const v
                                                          unsigned chunk, WorkItem *__restrict__ items,
                                                          unsigned long long cap, BatchCtl *ctl, BatchCtl *sctl,
                                                          const BatchCtl *prev, int req_base,
-                                                         nvshmemx_request *__restrict__ keep) {
+                                                         nvshmemx_request *__restrict__ keep, int *host) {
   __shared__ unsigned warp_sums[kPlanThreads / 32];
   __shared__ unsigned long long block_base;
   pdl_release_dependents();
   const unsigned long long ibase = prev ? prev->item_base + prev->total_chunks : 0ull;
+  if (prev && prev->status != 0) host = nullptr;  // the earlier piece's error is the one reported
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->item_base = ibase;
   const int i = blockIdx.x * kPlanThreads + threadIdx.x;
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -205,7 +214,7 @@ __global__ void __launch_bounds__(kPlanThreads) batch_plan_kernel(Cfg c, const v
     const nvshmemx_request r = load_request(reqs_in, i, COMPACT);
     if (COMPACT) store_request(keep + i, r);
     const int err = plan_one(c, r, chunk, w, cnt);
-    if (err) set_status(sctl, err, req_base + i);
+    if (err) set_status(sctl, err, req_base + i, host);
   }
   // CTA-wide exclusive scan of cnt
   unsigned incl = cnt;
@@ -224,7 +233,7 @@ __global__ void __launch_bounds__(kPlanThreads) batch_plan_kernel(Cfg c, const v
       acc += s;
     }
     block_base = acc ? atomicAdd(&ctl->total_chunks, (unsigned long long)acc) : 0ull;
-    if (acc && ibase + block_base + acc > cap) set_status(sctl, NVSHMEMX_ERR_NOMEM, -1);
+    if (acc && ibase + block_base + acc > cap) set_status(sctl, NVSHMEMX_ERR_NOMEM, -1, host);
   }
   __syncthreads();
   if (cnt == 0) return;
@@ -415,7 +424,7 @@ struct WarpTma {
 template <int S>
 __global__ void __launch_bounds__(256, 3) batch_exec_tma_kernel(const WorkItem *__restrict__ items, BatchCtl *ctl,
                                                               BatchCtl *sctl, unsigned long long cap, int grab,
-                                                              unsigned SB, unsigned min_bulk, long long timeout_ns) {
+                                                              unsigned SB, unsigned min_bulk, long long timeout_ns, int *host) {
   extern __shared__ __align__(128) char smem[];
   const unsigned lane = threadIdx.x & 31u;
   WarpTma<S> ring;
@@ -436,9 +445,7 @@ __global__ void __launch_bounds__(256, 3) batch_exec_tma_kernel(const WorkItem *
     for (unsigned long long k = bse; k < end; ++k) ring.run(load_item(items + k), lane);
     bse = __shfl_sync(0xffffffffu, nxt, 0);
   }
-  if (!ring.drain(lane) && lane == 0) {
-    if (atomicCAS(&sctl->status, 0, NVSHMEMX_ERR_TIMEOUT) == 0) sctl->bad_request = -2;
-  }
+  if (!ring.drain(lane) && lane == 0) set_status(sctl, NVSHMEMX_ERR_TIMEOUT, -2, host);
 }
 
 // ------------------------------------------------ small batches: one launch
@@ -791,19 +798,6 @@ __global__ void __launch_bounds__(256) batch_stream_kernel(Cfg c, const nvshmemx
   }
 }
 
-// End of a pipelined submit: once the last exec kernel is done (it lets this
-// kernel start early; griddepcontrol.wait holds it until the exec grid has
-// completed and its writes are visible), writes the batch status word and
-// the first bad request into the caller-visible pinned host words.
-__global__ void status_to_host_kernel(const BatchCtl *ctl, volatile int *host_status) {
-  pdl_wait_prerequisites();
-  if (threadIdx.x == 0) {
-    host_status[0] = *(volatile const int *)&ctl->status;
-    host_status[1] = *(volatile const int *)&ctl->bad_request;
-    __threadfence_system();
-  }
-}
-
 // Zeroes the control block of a streaming launch and moves its generation
 // on (one thread; a graph node in place of a memset).
 __global__ void stream_reset_kernel(StreamCtl *ctl) {
@@ -818,7 +812,7 @@ __global__ void stream_reset_kernel(StreamCtl *ctl) {
 }
 
 typedef void (*TmaFn)(const WorkItem *, BatchCtl *, BatchCtl *, unsigned long long, int, unsigned, unsigned,
-                      long long);
+                      long long, int *);
 
 static TmaFn pick_tma(int stages) {
   switch (stages) {
@@ -919,8 +913,8 @@ struct nvshmemx_batch {
   nvshmemx_batch_config cfg{};
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr;  // pipelined submit: copies and plans of the pieces
-  cudaEvent_t ev_reset = nullptr, ev_copied = nullptr;
-  cudaEvent_t ev_piece[3] = {nullptr, nullptr, nullptr};  // piece k planned
+  cudaEvent_t ev_reset = nullptr;
+  cudaEvent_t ev_piece[2] = {nullptr, nullptr};  // piece k planned
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   int graph_n = -1;
@@ -937,28 +931,19 @@ struct nvshmemx_batch {
   int last_pieces = 1;        // pieces of the last execution (pipelined submit: 2)
 };
 
-// Control block of piece k of a pipelined submit: bytes 0..31, 64..95 and
-// 96..127 of the batch's 128-byte control allocation (bytes 32..63 hold the
+// Control blocks: bytes 0..31 of the batch's control allocation for one piece,
+// 64..95 and 96..127 for the two of a pipelined submit (bytes 32..63 hold the
 // streaming generation, which must never be zeroed).
 static BatchCtl *piece_ctl(nvshmemx_batch *b, int k) {
-  static const int off[3] = {0, 64, 96};
-  return reinterpret_cast<BatchCtl *>(reinterpret_cast<char *>(b->d_ctl) + off[k]);
+  return reinterpret_cast<BatchCtl *>(reinterpret_cast<char *>(b->d_ctl) + 64 + 32 * k);
 }
 
-// Pieces of a pipelined submit (ends[k] = end of piece k, in requests): one
-// below 8192 requests, where the copy is too short to be worth hiding, else
-// two, a quarter (in whole 256-request plan blocks) and the rest.  (Three
-// pieces, an eighth / three eighths / a half, measured 6 us slower on the
-// 100,000-request batch: each extra exec launch costs more than it hides.)
-static int split_pieces(int n, int ends[3]) {
-  if (n < 8192) {
-    ends[0] = n;
-    return 1;
-  }
-  ends[0] = (n / 4) & ~255;
-  ends[1] = n;
-  return 2;
-}
+// From this many requests on a submit runs as two pieces, the first quarter
+// (in whole 256-request plan blocks) and the rest; below it the copy is too
+// short to be worth hiding.  (Three pieces, an eighth / three eighths / a half,
+// measured 6 us slower on the 100,000-request batch: each extra exec launch
+// costs more than it hides.)
+static const int kTwoPieces = 8192;
 
 static void drop_graph(nvshmemx_batch *b) {
   if (b->gexec) cudaGraphExecDestroy(b->gexec);
@@ -1001,7 +986,7 @@ static int enqueue_stream(nvshmemx_batch *b, bool with_events, const nvshmemx_re
 // b->d_reqs + req_base.
 enum { kPlan = 1, kExec = 2, kCompact = 4 };
 static int enqueue_piece(nvshmemx_batch *b, bool with_events, const void *src, int n, BatchCtl *ctl,
-                         BatchCtl *sctl, const BatchCtl *prev, int req_base, cudaStream_t st, int parts) {
+                         BatchCtl *sctl, const BatchCtl *prev, int req_base, cudaStream_t st, int parts, int *host) {
   const Runtime &r = rt();
   const Cfg c = r.cfg;
   const nvshmemx_batch_config &k = b->cfg;
@@ -1016,10 +1001,10 @@ static int enqueue_piece(nvshmemx_batch *b, bool with_events, const void *src, i
   if ((parts & kPlan) && n > 0) {
     if (parts & kCompact)
       batch_plan_kernel<true><<<(n + kPlanThreads - 1) / kPlanThreads, kPlanThreads, 0, st>>>(c, src, n, (unsigned)k.chunk_bytes, b->d_items, cap_end,
-                                                              ctl, sctl, prev, req_base, b->d_reqs + req_base);
+                                                              ctl, sctl, prev, req_base, b->d_reqs + req_base, host);
     else
       batch_plan_kernel<false><<<(n + kPlanThreads - 1) / kPlanThreads, kPlanThreads, 0, st>>>(c, src, n, (unsigned)k.chunk_bytes, b->d_items,
-                                                               cap_end, ctl, sctl, prev, req_base, nullptr);
+                                                               cap_end, ctl, sctl, prev, req_base, nullptr, host);
   }
   if (with_events) cudaEventRecord(b->ev_exec0, st);
   if (!(parts & kExec)) return check_cuda(cudaGetLastError(), "batch plan launch");
@@ -1052,7 +1037,7 @@ static int enqueue_piece(nvshmemx_batch *b, bool with_events, const void *src, i
   cudaError_t e;
   if (tfn)
     e = cudaLaunchKernelEx(&lc, tfn, (const WorkItem *)b->d_items, ctl, sctl, cap_end, k.grab,
-                           (unsigned)k.tma_stage_bytes, (unsigned)k.tma_min_bytes, (long long)c.wait_timeout_ns);
+                           (unsigned)k.tma_stage_bytes, (unsigned)k.tma_min_bytes, (long long)c.wait_timeout_ns, host);
   else
     e = cudaLaunchKernelEx(&lc, fn, (const WorkItem *)b->d_items, ctl, sctl, cap_end, k.grab);
   if (with_events) cudaEventRecord(b->ev_exec1, st);
@@ -1066,7 +1051,8 @@ static int enqueue_piece(nvshmemx_batch *b, bool with_events, const void *src, i
 static int enqueue_batch(nvshmemx_batch *b, bool with_events, const nvshmemx_request *src) {
   if (b->cfg.stream) return enqueue_stream(b, with_events, src);
   cudaMemsetAsync(b->d_ctl, 0, sizeof(BatchCtl), b->stream);
-  return enqueue_piece(b, with_events, src, b->n, b->d_ctl, b->d_ctl, nullptr, 0, b->stream, kPlan | kExec);
+  return enqueue_piece(b, with_events, src, b->n, b->d_ctl, b->d_ctl, nullptr, 0, b->stream, kPlan | kExec,
+                       b->h_status_dev);
 }
 
 static int ensure_graph(nvshmemx_batch *b, const nvshmemx_request *src) {
@@ -1206,7 +1192,7 @@ int batch_enqueue_range(nvshmemx_batch *b, int first, int n, const nvshmemx_batc
   const nvshmemx_batch_config saved = b->cfg;
   b->cfg = cfg;
   int rc = check_cuda(cudaMemsetAsync(b->d_ctl, 0, sizeof(BatchCtl), b->stream), "cudaMemsetAsync");
-  if (!rc) rc = enqueue_piece(b, false, b->d_reqs + first, n, b->d_ctl, b->d_ctl, nullptr, 0, b->stream, kPlan | kExec);
+  if (!rc) rc = enqueue_piece(b, false, b->d_reqs + first, n, b->d_ctl, b->d_ctl, nullptr, 0, b->stream, kPlan | kExec, nullptr);
   b->cfg = saved;
   if (!rc) {
     sticky_status_kernel<<<1, 32, 0, b->stream>>>(b->d_ctl, sticky_word(b));
@@ -1280,7 +1266,6 @@ int nvshmemx_batch_create(int max_requests, unsigned long long max_payload_bytes
   cudaEventCreate(&b->ev_exec0);
   cudaEventCreate(&b->ev_exec1);
   cudaEventCreateWithFlags(&b->ev_reset, cudaEventDisableTiming);
-  cudaEventCreateWithFlags(&b->ev_copied, cudaEventDisableTiming);
   for (auto &e : b->ev_piece) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
   void *hs = nullptr;
   if ((rc = check_cuda(cudaHostGetDevicePointer(&hs, b->h_status, 0), "cudaHostGetDevicePointer(status)"))) {
@@ -1308,7 +1293,7 @@ int nvshmemx_batch_destroy(nvshmemx_batch *b) {
   if (b->h_reqs) cudaFreeHost(b->h_reqs);
   if (b->h_status) cudaFreeHost(b->h_status);
   cudaEvent_t evs[] = {b->ev_start,    b->ev_stop,     b->ev_plan0,    b->ev_exec0,   b->ev_exec1,
-                       b->ev_reset,    b->ev_copied,   b->ev_piece[0], b->ev_piece[1], b->ev_piece[2]};
+                       b->ev_reset,    b->ev_piece[0], b->ev_piece[1]};
   for (auto e : evs)
     if (e) cudaEventDestroy(e);
   if (b->stream) cudaStreamDestroy(b->stream);
@@ -1362,91 +1347,90 @@ int nvshmemx_batch_execute(nvshmemx_batch *b, int reps, float *out_ms) {
   cudaEventElapsedTime(&ms, b->ev_start, b->ev_stop);
   if (out_ms) *out_ms = ms;
   int st[2] = {b->h_status[0], b->h_status[1]};
-  if (!small) cudaMemcpy(st, &b->d_ctl->status, sizeof st, cudaMemcpyDeviceToHost);
+  if (b->cfg.stream) cudaMemcpy(st, &b->d_ctl->status, sizeof st, cudaMemcpyDeviceToHost);
   if (st[0]) return fail(st[0], "batch_execute: request %d rejected (%s)", st[1], nvshmemx_strerror(st[0]));
   return 0;
 }
 
-// The pieces of a submit (graph configuration): see nvshmemx_batch_submit.
+// A submit of compact requests in one piece: copy, plan and exec in order on
+// the batch's stream.
+static int submit_one(nvshmemx_batch *b, const void *host, void *dev, size_t elem, int flag, int n) {
+  int rc;
+  b->last_pieces = 1;
+  b->h_status[0] = b->h_status[1] = 0;
+  if ((rc = check_cuda(cudaMemsetAsync(b->d_ctl, 0, sizeof(BatchCtl), b->stream), "cudaMemsetAsync")) ||
+      (rc = check_cuda(cudaMemcpyAsync(dev, host, (size_t)n * elem, cudaMemcpyHostToDevice, b->stream),
+                       "cudaMemcpyAsync(requests)")) ||
+      (rc = enqueue_piece(b, false, dev, n, b->d_ctl, b->d_ctl, nullptr, 0, b->stream, kPlan | kExec | flag,
+                          b->h_status_dev)))
+    cudaStreamSynchronize(b->stream);
+  return rc;
+}
+
+// A submit in two pieces (graph configuration): see nvshmemx_batch_submit.
 // `host` holds n requests of `elem` bytes (full or compact form, `flag` 0 or
-// kCompact), copied piece by piece to `dev`.
-static int submit_pieces(nvshmemx_batch *b, const void *host, void *dev, size_t elem, int flag, int pieces,
-                         const int ends[3]) {
+// kCompact), copied piece by piece to `dev`.  The copy stream copies and plans
+// the pieces in order (the second plan appends its items after the first's);
+// the batch's stream zeroes the control blocks beside the first copy and
+// executes each piece once it is planned.  Errors of either plan or exec reach
+// the pinned status words from the kernels themselves.  (Nothing of an earlier
+// call is on either stream: every call waits for its work.)
+static int submit_two(nvshmemx_batch *b, const void *host, void *dev, size_t elem, int flag, int n) {
+  const int ends[2] = {(n / 4) & ~255, n};
+  BatchCtl *c0 = piece_ctl(b, 0);
   int rc = 0;
-  // The copy stream copies and plans the pieces in order (each plan
-  // appends its items after the previous piece's); the batch's stream
-  // executes piece k once it is planned and piece k-1 has run.  Each piece
-  // has its own control block; the execs report into the first.
-  rc = check_cuda(cudaStreamWaitEvent(b->copy_stream, b->ev_start, 0), "cudaStreamWaitEvent");
-  if (!rc)
-    rc = check_cuda(cudaMemsetAsync(piece_ctl(b, 0), 0, sizeof(BatchCtl), b->copy_stream), "cudaMemsetAsync");
-  if (!rc)  // blocks 1 and 2 are contiguous (bytes 64..127)
-    rc = check_cuda(cudaMemsetAsync(piece_ctl(b, 1), 0, 2 * sizeof(BatchCtl), b->copy_stream), "cudaMemsetAsync");
-  for (int k = 0, at = 0; k < pieces && !rc; at = ends[k++]) {
+  b->last_pieces = 2;
+  b->h_status[0] = b->h_status[1] = 0;
+  for (int k = 0, at = 0; k < 2 && !rc; at = ends[k++]) {
     const int m = ends[k] - at;
     BatchCtl *ck = piece_ctl(b, k);
     const char *hsrc = static_cast<const char *>(host) + (size_t)at * elem;
     char *dsrc = static_cast<char *>(dev) + (size_t)at * elem;
     if ((rc = check_cuda(cudaMemcpyAsync(dsrc, hsrc, (size_t)m * elem, cudaMemcpyHostToDevice, b->copy_stream),
-                         "cudaMemcpyAsync(requests)")) ||
-        (rc = enqueue_piece(b, false, dsrc, m, ck, ck, k ? piece_ctl(b, k - 1) : nullptr, at, b->copy_stream,
-                            kPlan | flag)) ||
-        (rc = check_cuda(cudaEventRecord(b->ev_piece[k], b->copy_stream), "cudaEventRecord")))
+                         "cudaMemcpyAsync(requests)")))
       break;
-  }
-  for (int k = 0, at = 0; k < pieces && !rc; at = ends[k++]) {
-    if ((rc = check_cuda(cudaStreamWaitEvent(b->stream, b->ev_piece[k], 0), "cudaStreamWaitEvent")) ||
-        (rc = enqueue_piece(b, false, nullptr, ends[k] - at, piece_ctl(b, k), piece_ctl(b, 0), nullptr, at,
-                            b->stream, kExec)))
+    if (k == 0 && ((rc = check_cuda(cudaMemsetAsync(c0, 0, 2 * sizeof(BatchCtl), b->stream), "cudaMemsetAsync")) ||
+                   (rc = check_cuda(cudaEventRecord(b->ev_reset, b->stream), "cudaEventRecord")) ||
+                   (rc = check_cuda(cudaStreamWaitEvent(b->copy_stream, b->ev_reset, 0), "cudaStreamWaitEvent"))))
+      break;
+    if ((rc = enqueue_piece(b, false, dsrc, m, ck, ck, k ? c0 : nullptr, at, b->copy_stream, kPlan | flag,
+                            b->h_status_dev)) ||
+        (rc = check_cuda(cudaEventRecord(b->ev_piece[k], b->copy_stream), "cudaEventRecord")) ||
+        (rc = check_cuda(cudaStreamWaitEvent(b->stream, b->ev_piece[k], 0), "cudaStreamWaitEvent")) ||
+        (rc = enqueue_piece(b, false, nullptr, m, ck, c0, nullptr, at, b->stream, kExec, b->h_status_dev)))
       break;
   }
   if (rc) {
     cudaStreamSynchronize(b->copy_stream);
     cudaStreamSynchronize(b->stream);
-    return rc;
   }
-  BatchCtl *c0 = piece_ctl(b, 0);
-  // the status word reaches the host from a kernel that starts while the
-  // last exec runs and writes as soon as it is done (no copy to schedule)
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(1);
-  lc.blockDim = dim3(32);
-  lc.stream = b->stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  lc.attrs = attr;
-  lc.numAttrs = 1;
-  if ((rc = check_cuda(cudaLaunchKernelEx(&lc, status_to_host_kernel, (const BatchCtl *)c0,
-                                          (volatile int *)b->h_status_dev),
-                       "status kernel launch")))
-    return rc;
-  return 0;
+  return rc;
 }
 
 int nvshmemx_batch_submit(nvshmemx_batch *b, const nvshmemx_request *reqs, int n, int *out_status, float *out_ms) {
   if (!b || n < 0 || n > b->max_n || (n && !reqs)) return fail(NVSHMEMX_ERR_INVALID, "batch_submit: bad arguments");
   int rc;
   b->n = n;
-  int ends[3];
-  const bool small = small_batch(b, n);
-  const int pieces = b->cfg.stream ? 1 : split_pieces(n, ends);
-  if (!small && pieces == 1 && (rc = ensure_graph(b, b->d_reqs))) return rc;
-  b->last_pieces = pieces;
+  const bool small = small_batch(b, n), two = !b->cfg.stream && n >= kTwoPieces;
+  if (!small && !two && (rc = ensure_graph(b, b->d_reqs))) return rc;
+  b->last_pieces = 1;
   b->timed_direct = false;
-  cudaEventRecord(b->ev_start, b->stream);
+  b->h_status[0] = b->h_status[1] = 0;
+  cudaEventRecord(b->ev_start, two ? b->copy_stream : b->stream);
   if (small) {
     if ((rc = submit_small(b, reqs, b->d_reqs, sizeof(nvshmemx_request), false, n))) return rc;
-  } else if (pieces > 1) {
-    if ((rc = submit_pieces(b, reqs, b->d_reqs, sizeof(nvshmemx_request), 0, pieces, ends))) return rc;
+  } else if (two) {
+    if ((rc = submit_two(b, reqs, b->d_reqs, sizeof(nvshmemx_request), 0, n))) return rc;
   } else {
     if (n && (rc = check_cuda(cudaMemcpyAsync(b->d_reqs, reqs, (size_t)n * sizeof(nvshmemx_request),
                                               cudaMemcpyHostToDevice, b->stream),
                               "cudaMemcpyAsync(requests)")))
       return rc;
     if ((rc = check_cuda(cudaGraphLaunch(b->gexec, b->stream), "cudaGraphLaunch"))) return rc;
-    if ((rc = check_cuda(cudaMemcpyAsync(b->h_status, &b->d_ctl->status, 8, cudaMemcpyDeviceToHost, b->stream),
-                         "cudaMemcpyAsync(status)")))
+    // the streaming kernel keeps its status in device memory only
+    if (b->cfg.stream && (rc = check_cuda(cudaMemcpyAsync(b->h_status, &b->d_ctl->status, 8, cudaMemcpyDeviceToHost,
+                                                          b->stream),
+                                          "cudaMemcpyAsync(status)")))
       return rc;
   }
   cudaEventRecord(b->ev_stop, b->stream);
@@ -1472,15 +1456,13 @@ int nvshmemx_batch_submit_compact(nvshmemx_batch *b, const nvshmemx_request_comp
     b->last_pieces = 1;
     return 0;
   }
-  // every piece count goes through the copy stream: the plan kernels expand
-  // the compact requests and leave the full form in b->d_reqs
-  int ends[3];
-  const int pieces = split_pieces(n, ends);
-  b->last_pieces = pieces;
-  cudaEventRecord(b->ev_start, b->stream);
-  if (small_batch(b, n)) {
-    if ((rc = submit_small(b, reqs, b->d_reqs_compact, sizeof(nvshmemx_request_compact), true, n))) return rc;
-  } else if ((rc = submit_pieces(b, reqs, b->d_reqs_compact, sizeof(nvshmemx_request_compact), kCompact, pieces, ends)))
+  // the plan kernels expand the compact requests and leave the full form in
+  // b->d_reqs
+  const bool small = small_batch(b, n), two = n >= kTwoPieces;
+  cudaEventRecord(b->ev_start, two ? b->copy_stream : b->stream);
+  if ((rc = small ? submit_small(b, reqs, b->d_reqs_compact, sizeof(nvshmemx_request_compact), true, n)
+            : two ? submit_two(b, reqs, b->d_reqs_compact, sizeof(nvshmemx_request_compact), kCompact, n)
+                  : submit_one(b, reqs, b->d_reqs_compact, sizeof(nvshmemx_request_compact), kCompact, n)))
     return rc;
   cudaEventRecord(b->ev_stop, b->stream);
   if ((rc = check_cuda(cudaStreamSynchronize(b->stream), "batch_submit_compact"))) return rc;
@@ -1494,12 +1476,10 @@ int nvshmemx_batch_submit_compact(nvshmemx_batch *b, const nvshmemx_request_comp
 int nvshmemx_batch_last_stats(const nvshmemx_batch *b, unsigned long long *chunks, float *plan_ms, float *exec_ms) {
   if (!b) return NVSHMEMX_ERR_INVALID;
   if (chunks) {
-    BatchCtl h[4];  // bytes 0..127: piece 0, (streaming state), pieces 1 and 2
+    BatchCtl h[4];  // bytes 0..127: one piece, (streaming state), the two of a pipelined submit
     if (cudaMemcpy(h, b->d_ctl, sizeof h, cudaMemcpyDeviceToHost) != cudaSuccess)
       return check_cuda(cudaGetLastError(), "batch_last_stats");
-    *chunks = h[0].total_chunks;
-    if (b->last_pieces > 1) *chunks += h[2].total_chunks;
-    if (b->last_pieces > 2) *chunks += h[3].total_chunks;
+    *chunks = b->last_pieces > 1 ? h[2].total_chunks + h[3].total_chunks : h[0].total_chunks;
   }
   float p = 0, e = 0;
   if (b->timed_direct) {
@@ -1661,7 +1641,7 @@ extern "C" int nvshmemx_batch_execute_noalloc(const nvshmemx_request *d_reqs, in
   if ((rc = check_cuda(cudaMemsetAsync(ctl, 0, sizeof(BatchCtl), s), "cudaMemsetAsync(noalloc control)"))) return rc;
   if (n > 0)
     batch_plan_kernel<false><<<(n + kPlanThreads - 1) / kPlanThreads, kPlanThreads, 0, s>>>(r.cfg, d_reqs, n, (unsigned)k.chunk_bytes, items,
-                                                             kNoallocMaxItems, ctl, ctl, nullptr, 0, nullptr);
+                                                             kNoallocMaxItems, ctl, ctl, nullptr, 0, nullptr, nullptr);
   // The exec kernel the configuration names: TMA rings (their stages are
   // shared memory, not scratch) or the register copy.
   int per_sm = 0;
@@ -1681,7 +1661,7 @@ extern "C" int nvshmemx_batch_execute_noalloc(const nvshmemx_request *d_reqs, in
   if (tfn)
     tfn<<<r.sm_count * ctas, k.threads, smem, s>>>(items, ctl, ctl, kNoallocMaxItems, k.grab,
                                                     (unsigned)k.tma_stage_bytes, (unsigned)k.tma_min_bytes,
-                                                    (long long)r.cfg.wait_timeout_ns);
+                                                    (long long)r.cfg.wait_timeout_ns, nullptr);
   else
     fn<<<r.sm_count * ctas, k.threads, 0, s>>>(items, ctl, ctl, kNoallocMaxItems, k.grab);
   if ((rc = check_cuda(cudaGetLastError(), "batch_execute_noalloc launch"))) return rc;
