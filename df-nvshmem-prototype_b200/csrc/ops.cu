@@ -34,16 +34,57 @@ struct DevScratch {
 };
 static DevScratch g_req_buf, g_out_buf;
 
+// Times an operation on a stream with two events.  A host thread keeps its
+// pair from operation to operation (creating and destroying them cost a call
+// 3 us), one pair per thread, for the device that it last used.
 struct EventTimer {
+  struct Pair {
+    cudaEvent_t a = nullptr, b = nullptr;
+    int dev = -1;
+    bool busy = false;
+    void drop() {
+      if (a) cudaEventDestroy(a);
+      if (b) cudaEventDestroy(b);
+      a = b = nullptr;
+      dev = -1;
+    }
+    ~Pair() { drop(); }
+  };
+  static Pair &kept() {
+    static thread_local Pair p;
+    return p;
+  }
   cudaEvent_t a = nullptr, b = nullptr;
+  bool from_kept = false;
   EventTimer() {
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
+    Pair &p = kept();
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!p.busy) {
+      if (p.dev != dev) {
+        p.drop();
+        cudaEventCreate(&p.a);
+        cudaEventCreate(&p.b);
+        p.dev = dev;
+      }
+      p.busy = from_kept = true;
+      a = p.a;
+      b = p.b;
+    } else {
+      cudaEventCreate(&a);
+      cudaEventCreate(&b);
+    }
   }
   ~EventTimer() {
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
+    if (from_kept) {
+      kept().busy = false;
+    } else {
+      cudaEventDestroy(a);
+      cudaEventDestroy(b);
+    }
   }
+  EventTimer(const EventTimer &) = delete;
+  EventTimer &operator=(const EventTimer &) = delete;
   void start(cudaStream_t s = 0) { cudaEventRecord(a, s); }
   void stop(cudaStream_t s = 0) { cudaEventRecord(b, s); }
   float ms() {
@@ -92,7 +133,7 @@ __device__ __forceinline__ void copy_request(const Cfg &c, const nvshmemx_reques
                     (MODE == NVSHMEMX_MODE_WARP ? (threadIdx.x & 31) == 0 : threadIdx.x == 0));
   const unsigned long long t0 = rec ? gtimer() : 0;
   if (MODE == NVSHMEMX_MODE_THREAD)
-    copy_lanes<16, 8, true>(dst, src, bytes);
+    copy_lanes<16, 12, true>(dst, src, bytes);
   else if (MODE == NVSHMEMX_MODE_WARP)
     copy_warp<12>(dst, src, bytes, threadIdx.x & 31);
   else if (MODE == NVSHMEMX_MODE_BLOCK)
@@ -112,7 +153,7 @@ __device__ __forceinline__ void copy_request(const Cfg &c, const nvshmemx_reques
 // in CTAs of eight (its largest request, one warp's, is a third of that time).
 template <int MODE>
 __global__ void __launch_bounds__(MODE <= NVSHMEMX_MODE_WARP ? 64 : 256,
-                                  MODE == NVSHMEMX_MODE_THREAD ? 8 : MODE == NVSHMEMX_MODE_WARP ? 10 : 3)
+                                  MODE == NVSHMEMX_MODE_THREAD ? 6 : MODE == NVSHMEMX_MODE_WARP ? 10 : 3)
     exec_requests_kernel(Cfg c, const nvshmemx_request *__restrict__ reqs, int n, unsigned bulk_smem) {
   extern __shared__ __align__(128) char smem[];
   long long u;
@@ -295,18 +336,6 @@ __global__ void barrier_latency_kernel(int iters, int counted, long long *cycles
 }
 
 // -------------------------------------------------------------- C2 all-to-all
-// A CTA's share of one all-to-all round, [b, e) of the PE's (npes-1) *
-// `bytes` outgoing (put) or incoming (get) bytes, streamed by one thread
-// through one TMA ring of kA2aStages stages: the ring runs across message
-// boundaries, so a share that spans two messages is loaded and stored
-// without draining the ring between them (a cooperative bulk copy per
-// message fills and drains its ring once per message).  Every chunk stays
-// inside one message; all addresses are 16-byte aligned (the caller checks).
-// Shared memory: 8 mbarriers, the destination and length of each stage's
-// chunk (256 bytes), then the stages.  Stage reuse lags one store behind,
-// as in bulk_copy_1t.  Returns false if an mbarrier wait passed `deadline`.
-constexpr unsigned kA2aStages = 6;
-
 // Where message k of the share starts: its destination and source.
 __device__ __forceinline__ void a2a_message(const Cfg &c, int op, int pe, unsigned long long so, unsigned long long ro,
                                             unsigned long long bytes, unsigned long long k, char **dst,
@@ -321,78 +350,148 @@ __device__ __forceinline__ void a2a_message(const Cfg &c, int op, int pe, unsign
   }
 }
 
-// The issuing thread walks the share message by message (one division at
-// the start, none per chunk): a chunk costs it a few instructions, since at
-// tens of GB/s per CTA a 10 KiB chunk leaves it a few hundred cycles.
-__device__ __forceinline__ bool a2a_stream_1t(const Cfg &c, char *smem, unsigned smem_bytes, int op, int pe,
-                                              unsigned long long so, unsigned long long ro, unsigned long long bytes,
-                                              unsigned long long b, unsigned long long e,
-                                              unsigned long long deadline) {
-  if (b >= e) return true;
-  const unsigned S = kA2aStages;
-  unsigned long long *mbar = reinterpret_cast<unsigned long long *>(smem);
-  unsigned long long *sdst = reinterpret_cast<unsigned long long *>(smem + 64);
-  unsigned *slen = reinterpret_cast<unsigned *>(smem + 128);
-  char *buf = smem + 256;
-  const unsigned SB = ((smem_bytes - 256) / S) & ~127u;
-  for (unsigned s = 0; s < S; ++s) mbar_init(mbar + s, 1);
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  unsigned long long k = b / bytes, off = b - k * bytes, left = e - b;
+// A CTA's share of the all-to-all rounds: in each, [b, e) of the PE's (npes-1)
+// * `bytes` outgoing (put) or incoming (get) bytes, streamed by one thread
+// through one TMA ring of kA2aStages stages.  The ring runs across message
+// boundaries, so a share that spans two messages is loaded and stored without
+// draining the ring between them (a cooperative bulk copy per message fills
+// and drains its ring once per message), and, where no round's destinations
+// overlap any round's sources (`ahead`), across rounds: the loads of the next
+// round's first chunks are issued before this round's barrier, so a round no
+// longer starts by waiting for its first load (8 PEs, us a round with a ring
+// per round and now: 4 KiB messages 3.0 and 2.76, 256 KiB 8.2 and 7.2, 1 MiB
+// 21.6 and 20.9).  Every chunk stays inside one message; all addresses are 16-byte aligned (the
+// caller checks).  Stage reuse lags one store behind, as in bulk_copy_1t.
+// Shared memory: 8 mbarriers, the destination and length of each stage's chunk
+// (256 bytes), then the stages.
+constexpr unsigned kA2aStages = 6;
+constexpr unsigned kLastOfRound = 1u << 31;  // in a stage's length: the share's last chunk
+
+struct A2aRing {
+  unsigned long long *mbar, *sdst;
+  unsigned *slen;
+  char *buf;
+  unsigned SB;
+  unsigned issued, stored;       // chunks loaded and stored so far, over all rounds
+  // the next chunk to load: in round `lr`, at `off` of message k, `left` bytes
+  // of the round's share from there
+  int lr;
+  unsigned long long k, off, left;
   char *dbase;
   const char *sbase;
-  a2a_message(c, op, pe, so, ro, bytes, k, &dbase, &sbase);
-  unsigned issued = 0, stored = 0;
-  while (issued < S && left) {
-    unsigned long long len = bytes - off;
-    if (len > left) len = left;
-    if (len > SB) len = SB;
-    sdst[issued] = (unsigned long long)(dbase + off);
-    slen[issued] = (unsigned)len;
-    mbar_expect_tx(mbar + issued, (unsigned)len);
-    bulk_g2s(buf + (size_t)issued * SB, sbase + off, (unsigned)len, mbar + issued);
-    ++issued;
-    off += len;
-    left -= len;
-    if (off == bytes && left) {
-      off = 0;
-      a2a_message(c, op, pe, so, ro, bytes, ++k, &dbase, &sbase);
-    }
+};
+
+// The share and the buffers it moves between (the same for every round).
+struct A2aShare {
+  int op, pe, nsets;
+  unsigned long long send, recv, stride, bytes, b, e;
+};
+
+__device__ __forceinline__ void a2a_round_start(const Cfg &c, A2aRing &g, const A2aShare &h, int round) {
+  const unsigned long long set = (unsigned long long)(round % h.nsets) * h.stride;
+  g.lr = round;
+  g.k = h.b / h.bytes;
+  g.off = h.b - g.k * h.bytes;
+  g.left = h.e - h.b;
+  a2a_message(c, h.op, h.pe, h.send + set, h.recv + set, h.bytes, g.k, &g.dbase, &g.sbase);
+}
+
+// Loads the next chunk into the next stage (which must be free).  The issuing
+// thread walks the share message by message (one division per round, none per
+// chunk): at tens of GB/s per CTA a 10 KiB chunk leaves it a few hundred cycles.
+__device__ __forceinline__ void a2a_load(const Cfg &c, A2aRing &g, const A2aShare &h) {
+  unsigned long long len = h.bytes - g.off;
+  if (len > g.left) len = g.left;
+  if (len > g.SB) len = g.SB;
+  const unsigned s = g.issued % kA2aStages;
+  g.sdst[s] = (unsigned long long)(g.dbase + g.off);
+  g.slen[s] = (unsigned)len | (g.left == len ? kLastOfRound : 0u);
+  mbar_expect_tx(g.mbar + s, (unsigned)len);
+  bulk_g2s(g.buf + (size_t)s * g.SB, g.sbase + g.off, (unsigned)len, g.mbar + s);
+  ++g.issued;
+  g.off += len;
+  g.left -= len;
+  if (g.off == h.bytes && g.left) {
+    const unsigned long long set = (unsigned long long)(g.lr % h.nsets) * h.stride;
+    g.off = 0;
+    a2a_message(c, h.op, h.pe, h.send + set, h.recv + set, h.bytes, ++g.k, &g.dbase, &g.sbase);
   }
-  bool ok = true;
-  while (stored < issued) {
-    const unsigned s = stored % S;
-    if (!mbar_wait(mbar + s, (stored / S) & 1u, deadline)) {
-      ok = false;
-      break;
+}
+
+// One thread: the stores of round `round`, with loads running ahead up to the
+// end of round `last_load`.  Returns false if an mbarrier wait passed
+// `deadline`; every store it issued is complete when it returns.
+__device__ __forceinline__ bool a2a_round_1t(const Cfg &c, A2aRing &g, const A2aShare &h, int round, int last_load,
+                                             unsigned long long deadline) {
+  auto more = [&]() -> bool {
+    if (g.left == 0 && g.lr < last_load) a2a_round_start(c, g, h, g.lr + 1);
+    return g.left != 0;
+  };
+  if (g.lr < round) a2a_round_start(c, g, h, round);
+  while (g.issued - g.stored < kA2aStages && more()) a2a_load(c, g, h);
+  bool last = false;
+  for (unsigned i = 0; !last; ++i) {
+    const unsigned s = g.stored % kA2aStages;
+    if (!mbar_wait(g.mbar + s, (g.stored / kA2aStages) & 1u, deadline)) {
+      bulk_wait_all();
+      return false;
     }
-    bulk_s2g(reinterpret_cast<void *>(sdst[s]), buf + (size_t)s * SB, slen[s]);
+    const unsigned len = g.slen[s];
+    last = (len & kLastOfRound) != 0;
+    bulk_s2g(reinterpret_cast<void *>(g.sdst[s]), g.buf + (size_t)s * g.SB, len & ~kLastOfRound);
     bulk_commit();
+    ++g.stored;
     // refill the stage the previous store read, not this one (see bulk_copy_1t)
-    if (stored >= 1 && left) {
+    if (i >= 1 && more()) {
       bulk_wait_read1();
-      const unsigned ps = (stored - 1) % S;
-      unsigned long long len = bytes - off;
-      if (len > left) len = left;
-      if (len > SB) len = SB;
-      sdst[ps] = (unsigned long long)(dbase + off);
-      slen[ps] = (unsigned)len;
-      mbar_expect_tx(mbar + ps, (unsigned)len);
-      bulk_g2s(buf + (size_t)ps * SB, sbase + off, (unsigned)len, mbar + ps);
-      ++issued;
-      off += len;
-      left -= len;
-      if (off == bytes && left) {
-        off = 0;
-        a2a_message(c, op, pe, so, ro, bytes, ++k, &dbase, &sbase);
-      }
+      a2a_load(c, g, h);
     }
-    ++stored;
   }
   bulk_wait_all();
-  if (ok)
-    for (unsigned s = 0; s < S; ++s) mbar_inval(mbar + s);
-  return ok;
+  // every stage is free now: the next round's loads pass the barrier
+  while (g.issued - g.stored < kA2aStages && more()) a2a_load(c, g, h);
+  return true;
+}
+
+// Rounds in the CTA-wide TMA mode when everything is 16-byte aligned: a
+// kernel of its own, so that the ring's state has the registers (in one kernel
+// with the unaligned copies it spilled, which cost 1.1 us a round).
+__global__ void __launch_bounds__(256, 3) alltoall_ring_kernel(Cfg c, A2aShare share, int rounds, unsigned bulk_smem,
+                                                               int device_barrier, int ahead) {
+  extern __shared__ __align__(128) char smem[];
+  const unsigned long long total = (unsigned long long)(c.npes - 1) * share.bytes;
+  const unsigned long long seg = (((total + gridDim.x - 1) / gridDim.x) + 15) & ~15ull;
+  share.pe = blockIdx.z;
+  share.b = blockIdx.x * seg;
+  share.e = share.b + seg < total ? share.b + seg : total;
+  A2aRing ring;
+  ring.mbar = reinterpret_cast<unsigned long long *>(smem);
+  ring.sdst = reinterpret_cast<unsigned long long *>(smem + 64);
+  ring.slen = reinterpret_cast<unsigned *>(smem + 128);
+  ring.buf = smem + 256;
+  ring.SB = ((bulk_smem - 256) / kA2aStages) & ~127u;
+  ring.issued = ring.stored = 0;
+  ring.lr = -1;
+  ring.left = 0;
+  bool run = threadIdx.x == 0 && share.b < share.e;
+  if (run) {
+    for (unsigned s = 0; s < kA2aStages; ++s) mbar_init(ring.mbar + s, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  for (int r = 0; r < rounds; ++r) {
+    if (run && !a2a_round_1t(c, ring, share, r, ahead && r + 1 < rounds ? r + 1 : r,
+                             gtimer() + (unsigned long long)c.wait_timeout_ns)) {
+      record_error(c, NVSHMEMX_ERR_TIMEOUT, -2);
+      run = false;
+    }
+    if (device_barrier) {
+      nvshmemx_barrier_all_ep((unsigned long long)r);
+    } else {
+      __syncthreads();
+      if (threadIdx.x == 0) nvshmem_quiet();
+    }
+  }
 }
 
 // Message k (0..npes-2) of PE p goes to / comes from peer q = (p+1+k) % npes.
@@ -400,10 +499,14 @@ __device__ __forceinline__ bool a2a_stream_1t(const Cfg &c, char *smem, unsigned
 // contiguous, 16-byte-rounded segment per caller unit (warp or CTA), so every
 // unit streams one range; MODE_THREAD keeps the prototype's shape, one thread
 // per message through the typed per-thread call.
-// Bounds: as many threads and CTAs per SM as its callers may ask for (a thread
-// per message up to 289 PEs; two, with the ring's shared memory three, CTAs).
+// Bounds: as many threads and CTAs per SM as its callers may ask for (kThreadMany:
+// a thread per message up to 289 PEs; two CTAs, with the ring's shared memory
+// three).
+constexpr int kThreadMany = 4;  // MODE_THREAD for more than 33 PEs
+
 template <int MODE>
-__global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 288 : 256, MODE == NVSHMEMX_MODE_BULK ? 3 : 2)
+__global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 32 : MODE == kThreadMany ? 288 : 256,
+                                  MODE == NVSHMEMX_MODE_BULK ? 3 : 2)
     alltoall_kernel(Cfg c, int op, int dtype, unsigned long long send_off,
                                 unsigned long long recv_off, unsigned long long bytes, int rounds, int nsets,
                                 unsigned long long set_stride, unsigned bulk_smem, int device_barrier) {
@@ -411,7 +514,8 @@ __global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 288 : 256, MODE
   const int pe = blockIdx.z, np = c.npes;
   const unsigned long long total = (unsigned long long)(np - 1) * bytes;
   unsigned long long unit, nunits;
-  if (MODE == NVSHMEMX_MODE_THREAD) {
+  constexpr bool by_thread = MODE == NVSHMEMX_MODE_THREAD || MODE == kThreadMany;
+  if (by_thread) {
     unit = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
     nunits = (unsigned long long)(np - 1);
   } else if (MODE == NVSHMEMX_MODE_WARP) {
@@ -421,10 +525,11 @@ __global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 288 : 256, MODE
     unit = blockIdx.x;
     nunits = gridDim.x;
   }
+  const unsigned long long seg = (((total + nunits - 1) / nunits) + 15) & ~15ull;  // a unit's share of a round
   for (int r = 0; r < rounds; ++r) {
     const unsigned long long so = send_off + (unsigned long long)(r % nsets) * set_stride;
     const unsigned long long ro = recv_off + (unsigned long long)(r % nsets) * set_stride;
-    if (MODE == NVSHMEMX_MODE_THREAD) {
+    if (by_thread) {
       // the copies of nvshmem_{T}_put / _get by one thread per message; the
       // lanes without a message help (copy_lanes)
       char *dst = nullptr;
@@ -433,21 +538,12 @@ __global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 288 : 256, MODE
       if (mine) a2a_message(c, op, pe, so, ro, bytes, unit, &dst, &src);
       const bool rec = mine && c.trace;
       const unsigned long long t0 = rec ? gtimer() : 0;
-      copy_lanes<8, 4, true>(dst, src, mine ? bytes : 0);
+      copy_lanes<8, MODE == NVSHMEMX_MODE_THREAD ? 8 : 4, true>(dst, src, mine ? bytes : 0);
       if (rec)
         trace_rec(c, (op == NVSHMEMX_REQ_PUT ? NVSHMEMX_TRACE_PUT_INT : NVSHMEMX_TRACE_GET_INT) + dtype,
                   op == NVSHMEMX_REQ_PUT ? src : dst, op == NVSHMEMX_REQ_PUT ? dst : src, bytes,
                   (pe + 1 + (int)unit) % np, t0, gtimer());
-    } else if (MODE == NVSHMEMX_MODE_BULK && ((bytes | so | ro) & 15) == 0) {
-      // one ring per CTA across its whole share of the round
-      const unsigned long long seg = (((total + nunits - 1) / nunits) + 15) & ~15ull;
-      const unsigned long long b = unit * seg;
-      const unsigned long long e = b + seg < total ? b + seg : total;
-      if (threadIdx.x == 0 && b < e &&
-          !a2a_stream_1t(c, smem, bulk_smem, op, pe, so, ro, bytes, b, e, gtimer() + (unsigned long long)c.wait_timeout_ns))
-        record_error(c, NVSHMEMX_ERR_TIMEOUT, -2);
     } else {
-      const unsigned long long seg = (((total + nunits - 1) / nunits) + 15) & ~15ull;
       unsigned long long b = unit * seg;
       const unsigned long long e = b + seg < total ? b + seg : total;
       while (b < e) {
@@ -474,11 +570,14 @@ __global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 288 : 256, MODE
         b += len;
       }
     }
-    // quiet + barrier: the barrier's __syncthreads orders every thread's
-    // stores before the leader, whose quiet and release cover them all
-    __syncthreads();
-    if (threadIdx.x == 0) nvshmem_quiet();
-    if (device_barrier) nvshmemx_barrier_all_ep((unsigned long long)r);
+    // the barrier's __syncthreads orders every thread's stores before the
+    // leader, whose release (without a barrier: quiet) covers them all
+    if (device_barrier) {
+      nvshmemx_barrier_all_ep((unsigned long long)r);
+    } else {
+      __syncthreads();
+      if (threadIdx.x == 0) nvshmem_quiet();
+    }
   }
 }
 
@@ -897,15 +996,42 @@ static int alltoall_setup(int op, int dtype, size_t send_off, size_t recv_off, s
   *block = dim3(256);
   switch (mode) {
     case NVSHMEMX_MODE_THREAD:
-      *fn = (const void *)alltoall_kernel<NVSHMEMX_MODE_THREAD>;
+      // one warp holds the messages of up to 33 PEs: its kernel has the
+      // registers for 8 vectors in flight per lane (7 messages of 4 KiB 4.8 us a
+      // round, 11 us with the 4 of the kernel for more PEs, 7.9 us with every
+      // message copied by one lane)
+      *fn = r.npes <= 33 ? (const void *)alltoall_kernel<NVSHMEMX_MODE_THREAD>
+                         : (const void *)alltoall_kernel<kThreadMany>;
       *grid = dim3(1);
       *block = dim3(32 * ((r.npes - 1 + 31) / 32));
       break;
     case NVSHMEMX_MODE_WARP: *fn = (const void *)alltoall_kernel<NVSHMEMX_MODE_WARP>; break;
     case NVSHMEMX_MODE_BLOCK: *fn = (const void *)alltoall_kernel<NVSHMEMX_MODE_BLOCK>; break;
-    default: *fn = (const void *)alltoall_kernel<NVSHMEMX_MODE_BULK>;
+    default: {
+      // the ring that runs across rounds needs every buffer 16-byte aligned
+      const bool aligned = ((bytes | send_off | recv_off | (nsets > 1 ? set_stride : 0)) & 15) == 0;
+      *fn = aligned ? (const void *)alltoall_ring_kernel : (const void *)alltoall_kernel<NVSHMEMX_MODE_BULK>;
+    }
   }
   return 0;
+}
+
+// One collective launch of `rounds` rounds from buffer sets at send / recv.
+static int alltoall_launch(const void *fn, dim3 grid, dim3 block, unsigned smem, int op, int dtype, size_t send,
+                           size_t recv, size_t bytes, int rounds, int nsets, size_t stride, int device_barrier) {
+  Cfg c = rt().cfg;
+  unsigned long long so = send, ro = recv, by = bytes, ss = stride;
+  if (fn != (const void *)alltoall_ring_kernel) {
+    void *args[] = {&c, &op, &dtype, &so, &ro, &by, &rounds, &nsets, &ss, &smem, &device_barrier};
+    return launch_collective(fn, grid, block, args, smem, 0);
+  }
+  A2aShare share = {op, 0, nsets, so, ro, ss, by, 0, 0};
+  // a round's sources may be read before the round in front of it is over when
+  // no round writes them: the send and receive buffers lie apart
+  const size_t span = (size_t)(nsets - 1) * stride + (size_t)rt().npes * bytes;
+  int ahead = send + span <= recv || recv + span <= send;
+  void *args[] = {&c, &share, &rounds, &smem, &device_barrier, &ahead};
+  return launch_collective(fn, grid, block, args, smem, 0);
 }
 
 int nvshmemx_op_alltoall(int op, int dtype, size_t send_off, size_t recv_off, size_t bytes, int rounds, int nsets,
@@ -917,13 +1043,10 @@ int nvshmemx_op_alltoall(int op, int dtype, size_t send_off, size_t recv_off, si
   if ((rc = alltoall_setup(op, dtype, send_off, recv_off, bytes, rounds, nsets, set_stride, mode, ctas_per_pe, &fn,
                            &grid, &block, &smem)))
     return rc;
-  Cfg c = rt().cfg;
-  unsigned long long so = send_off, ro = recv_off, by = bytes, ss = set_stride;
-  int device_barrier = 1;
-  void *args[] = {&c, &op, &dtype, &so, &ro, &by, &rounds, &nsets, &ss, &smem, &device_barrier};
   EventTimer t;
   t.start();
-  if ((rc = launch_collective(fn, grid, block, args, smem, 0))) return rc;
+  if ((rc = alltoall_launch(fn, grid, block, smem, op, dtype, send_off, recv_off, bytes, rounds, nsets, set_stride, 1)))
+    return rc;
   t.stop();
   float ms = t.ms();
   if (out_ms) *out_ms = ms;
@@ -939,16 +1062,12 @@ int nvshmemx_op_alltoall_host(int op, int dtype, size_t send_off, size_t recv_of
   if ((rc = alltoall_setup(op, dtype, send_off, recv_off, bytes, rounds, nsets, set_stride, mode, ctas_per_pe, &fn,
                            &grid, &block, &smem)))
     return rc;
-  Cfg c = rt().cfg;
-  unsigned long long by = bytes, ss = 0;
-  int one = 1, device_barrier = 0;
   EventTimer t;
   t.start();
   for (int rd = 0; rd < rounds; ++rd) {
-    unsigned long long so = send_off + (size_t)(rd % nsets) * set_stride;
-    unsigned long long ro = recv_off + (size_t)(rd % nsets) * set_stride;
-    void *args[] = {&c, &op, &dtype, &so, &ro, &by, &one, &one, &ss, &smem, &device_barrier};
-    if ((rc = launch_collective(fn, grid, block, args, smem, 0))) return rc;
+    const size_t set = (size_t)(rd % nsets) * set_stride;
+    if ((rc = alltoall_launch(fn, grid, block, smem, op, dtype, send_off + set, recv_off + set, bytes, 1, 1, 0, 0)))
+      return rc;
     nvshmem_barrier_all();
     if ((rc = last_launch("alltoall_host round"))) return rc;
   }

@@ -70,3 +70,37 @@ def test_thread_form_in_an_all_to_all_of_odd_messages(shmem_factory):
         sh.alltoall(REQ_GET, DT_INT, 0, 1 << 19, nbytes, rounds=2, mode=mode, ctas_per_pe=2)
     om.alltoall(1, 0, 1 << 19, nbytes, rounds=1)
     assert np.array_equal(heap_images(sh, npes, 1 << 20), om.heap)
+
+
+@pytest.mark.parametrize("op", [REQ_PUT, REQ_GET])
+@pytest.mark.parametrize("nbytes,ctas", [(16, 3), (64, 1), (10 * 1024, 2), (64 * 1024 + 16, 1), (100_000, 5)])
+@pytest.mark.parametrize("apart", [True, False])
+def test_ring_across_rounds(shmem_factory, op, nbytes, ctas, apart):
+    """Rounds of the CTA-wide TMA mode over rotating buffer sets: shares below a
+    chunk, of several messages and of more chunks than the ring has stages;
+    with receive buffers that a later round sends from again (`apart` false),
+    where no load may pass a barrier."""
+    npes, nsets, rounds = 5, 3, 7
+    one = (npes * nbytes + 15) // 16 * 16
+    heap = 8 << 20
+    recv = 4 << 20 if apart else one  # set s is received where set s + 1 is sent from
+    sh, om = shmem_factory(npes, heap), Model(npes, heap)
+    for pe in range(npes):
+        sh.fill_random(pe, 0, heap, 8)
+        om.fill_random(pe, 0, heap, 8)
+    sh.alltoall(op, DT_INT, 0, recv, nbytes, rounds=rounds, nsets=nsets, set_stride=one, mode=MODE_BULK,
+                ctas_per_pe=ctas)
+    assert sh.status() == 0
+    om.alltoall(1 if op == REQ_GET else 0, 0, recv, nbytes, rounds=rounds, nsets=nsets, set_stride=one)
+    assert np.array_equal(heap_images(sh, npes, heap), om.heap)
+
+
+def test_all_to_all_by_threads_of_several_warps(shmem_factory):
+    npes, nbytes, heap = 40, 1028, 256 << 10
+    sh, om = shmem_factory(npes, heap), Model(npes, heap)
+    for pe in range(npes):
+        sh.fill_random(pe, 0, heap, 9)
+        om.fill_random(pe, 0, heap, 9)
+    sh.alltoall(REQ_PUT, DT_INT, 0, 128 << 10, nbytes, rounds=2, mode=MODE_THREAD)
+    om.alltoall(0, 0, 128 << 10, nbytes, rounds=2)
+    assert np.array_equal(heap_images(sh, npes, heap), om.heap)
