@@ -151,9 +151,22 @@ __device__ __forceinline__ void copy_request(const Cfg &c, const nvshmemx_reques
 // work.  The warp form runs 20 warps per SM with 12 vectors in flight each:
 // 100,000 requests 255-270 us, against 300-360 us with 24 warps of 8 vectors
 // in CTAs of eight (its largest request, one warp's, is a third of that time).
-template <int MODE>
-__global__ void __launch_bounds__(MODE <= NVSHMEMX_MODE_WARP ? 64 : 256,
-                                  MODE == NVSHMEMX_MODE_THREAD ? 6 : MODE == NVSHMEMX_MODE_WARP ? 10 : 3)
+//
+// The CTA forms have two shapes.  A CTA spends about 2 us on a short request
+// (its descriptor, then its data), so many requests want many CTAs: 128 threads,
+// seven to an SM (block form, 100,000 requests of median 2 KiB 505 -> 291 us,
+// 20,000 125 -> 93 us; TMA form 510 -> 308 us and 126 -> 100 us).  With fewer
+// the longest requests decide, and three CTAs of 256 threads are ahead (block
+// form, 1500 requests of median 64 KiB 110 against 122 us, 4100 of 16 KiB 107
+// against 113; the TMA form, whose ring shrinks with the CTA, 6000 of 16 KiB
+// 121 against 139 us).
+constexpr int kManyBlock = 6144, kManyBulk = 12288;
+
+template <int MODE, int THREADS>
+__global__ void __launch_bounds__(THREADS, MODE == NVSHMEMX_MODE_THREAD ? 6
+                                           : MODE == NVSHMEMX_MODE_WARP ? 10
+                                           : THREADS == 128             ? 7
+                                                                        : 3)
     exec_requests_kernel(Cfg c, const nvshmemx_request *__restrict__ reqs, int n, unsigned bulk_smem) {
   extern __shared__ __align__(128) char smem[];
   long long u;
@@ -898,6 +911,9 @@ static unsigned halo_smem(int n) { return halo_rows(n) ? 128 + 8 * kHaloStage : 
 // Shared memory for the CTA-wide TMA copies: a 64 KiB ring (six stages)
 // plus 128 bytes of mbarriers (three CTAs fit an SM).
 static const unsigned kBulkSmem = 4 * 16384 + 128;
+// ... and the ring of the CTAs of 128 threads (exec_requests_kernel): seven
+// CTAs fit an SM.
+static const unsigned kBulkSmemMany = 30 * 1024 + 128;
 
 namespace nvshm {
 int launch_exec_requests(int mode, const nvshmemx_request *dr, int n, cudaStream_t s) {
@@ -905,18 +921,24 @@ int launch_exec_requests(int mode, const nvshmemx_request *dr, int n, cudaStream
   if (n <= 0) return 0;
   switch (mode) {
     case NVSHMEMX_MODE_THREAD:
-      exec_requests_kernel<NVSHMEMX_MODE_THREAD><<<(n + 63) / 64, 64, 0, s>>>(c, dr, n, 0);
+      exec_requests_kernel<NVSHMEMX_MODE_THREAD, 64><<<(n + 63) / 64, 64, 0, s>>>(c, dr, n, 0);
       break;
     case NVSHMEMX_MODE_WARP:
-      exec_requests_kernel<NVSHMEMX_MODE_WARP><<<(n + 1) / 2, 64, 0, s>>>(c, dr, n, 0);
+      exec_requests_kernel<NVSHMEMX_MODE_WARP, 64><<<(n + 1) / 2, 64, 0, s>>>(c, dr, n, 0);
       break;
     case NVSHMEMX_MODE_BLOCK:
-      exec_requests_kernel<NVSHMEMX_MODE_BLOCK><<<n, 256, 0, s>>>(c, dr, n, 0);
+      if (n > kManyBlock)
+        exec_requests_kernel<NVSHMEMX_MODE_BLOCK, 128><<<n, 128, 0, s>>>(c, dr, n, 0);
+      else
+        exec_requests_kernel<NVSHMEMX_MODE_BLOCK, 256><<<n, 256, 0, s>>>(c, dr, n, 0);
       break;
-    default:
-      cudaFuncSetAttribute(exec_requests_kernel<NVSHMEMX_MODE_BULK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)kBulkSmem);
-      exec_requests_kernel<NVSHMEMX_MODE_BULK><<<n, 256, kBulkSmem, s>>>(c, dr, n, kBulkSmem);
+    default: {
+      const bool many = n > kManyBulk;
+      const auto fn = many ? exec_requests_kernel<NVSHMEMX_MODE_BULK, 128> : exec_requests_kernel<NVSHMEMX_MODE_BULK, 256>;
+      const unsigned smem = many ? kBulkSmemMany : kBulkSmem;
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      fn<<<n, many ? 128 : 256, smem, s>>>(c, dr, n, smem);
+    }
   }
   return check_cuda(cudaGetLastError(), "exec_requests launch");
 }

@@ -104,3 +104,24 @@ def test_all_to_all_by_threads_of_several_warps(shmem_factory):
     sh.alltoall(REQ_PUT, DT_INT, 0, 128 << 10, nbytes, rounds=2, mode=MODE_THREAD)
     om.alltoall(0, 0, 128 << 10, nbytes, rounds=2)
     assert np.array_equal(heap_images(sh, npes, heap), om.heap)
+
+
+@pytest.mark.parametrize("mode,n", [(MODE_BLOCK, 6145), (MODE_BULK, 12289)])
+def test_cta_forms_with_many_requests(shmem_factory, mode, n):
+    """From here on the CTA forms run with 128 threads to a CTA."""
+    sh, om = shmem_factory(2, HEAP), Model(2, HEAP)
+    for pe in range(2):
+        sh.fill_random(pe, 0, HEAP, 10)
+        om.fill_random(pe, 0, HEAP, 10)
+    sizes = [4, 100, 1000, 2052] * (n // 4) + [70_004]
+    rows, at = [], HEAP // 2
+    for k, nb in enumerate(sizes):
+        rows.append(dict(src_off=(k * 64) % 4_000_000 + 4 * (k % 4), dst_off=at, bytes=nb, src_pe=k % 2,
+                         dst_pe=(k // 2) % 2, op=REQ_PUT if k % 2 else REQ_GET, dtype=DT_INT))
+        at += (nb + 15) // 16 * 16
+    assert len(rows) == n and at <= HEAP
+    reqs = requests(rows)
+    sh.exec_requests(reqs, mode)
+    assert sh.status() == 0
+    om.apply_requests(reqs)
+    assert first_diff(heap_images(sh, 2, HEAP), om.heap) is None
