@@ -193,6 +193,7 @@ __device__ __forceinline__ void store_request(nvshmemx_request *p, const nvshmem
 // the same C4 step (206.5-206.8 us) and end-to-end call (237.9-239.6 us), so
 // the contention of those atomics is not what the plan kernel waits on.
 constexpr int kPlanThreads = 256;
+constexpr unsigned kOwnChunks = 4;
 
 template <bool COMPACT>
 __global__ void __launch_bounds__(kPlanThreads) batch_plan_kernel(Cfg c, const void *__restrict__ reqs_in, int n,
@@ -209,7 +210,7 @@ __global__ void __launch_bounds__(kPlanThreads) batch_plan_kernel(Cfg c, const v
   const int i = blockIdx.x * kPlanThreads + threadIdx.x;
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   unsigned cnt = 0;
-  WorkItem w;
+  WorkItem w = {};
   if (i < n) {
     const nvshmemx_request r = load_request(reqs_in, i, COMPACT);
     if (COMPACT) store_request(keep + i, r);
@@ -236,10 +237,27 @@ __global__ void __launch_bounds__(kPlanThreads) batch_plan_kernel(Cfg c, const v
     if (acc && ibase + block_base + acc > cap) set_status(sctl, NVSHMEMX_ERR_NOMEM, -1, host);
   }
   __syncthreads();
-  if (cnt == 0) return;
+  // A thread writes the chunks of a short request itself; those of a long one
+  // are written by its warp together (one thread took longer over the chunks of
+  // the largest request than the rest of the kernel: 25,000 requests executed
+  // again 78.1 -> 75.4 us a call).
   const unsigned long long first = ibase + block_base + warp_sums[warp] + (incl - cnt);
-  if (first + cnt > cap) return;
-  for (unsigned k = 0; k < cnt; ++k) items[first + k] = chunk_of(w, k, chunk);
+  const bool fits = cnt != 0 && first + cnt <= cap;
+  const bool own = fits && cnt <= kOwnChunks;
+  for (unsigned k = 0; own && k < cnt; ++k) items[first + k] = chunk_of(w, k, chunk);
+  for (unsigned todo = __ballot_sync(0xffffffffu, fits && !own); todo; todo &= todo - 1) {
+    const int o = __ffs(todo) - 1;
+    WorkItem v;
+    v.dst = __shfl_sync(0xffffffffu, w.dst, o);
+    v.src = __shfl_sync(0xffffffffu, w.src, o);
+    v.len = __shfl_sync(0xffffffffu, w.len, o);
+    v.kind = kCopy;
+    v.value = 0;
+    v.pad = 0;
+    const unsigned long long at = __shfl_sync(0xffffffffu, first, o);
+    const unsigned m = __shfl_sync(0xffffffffu, cnt, o);
+    for (unsigned k = lane; k < m; k += 32) items[at + k] = chunk_of(v, k, chunk);
+  }
 }
 
 // ------------------------------------------------------------------- exec
