@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(256, 3) batch_exec_tma_kernel(const WorkItem *
 // SM (with 16 KiB chunks a 64-request batch keeps some 80 of 1184 warps
 // busy).  CTA b takes pieces b, b + gridDim.x, ..., its warps the next one
 // each.  Measured per call from pinned memory: 64 requests 49 -> 29 us, 1000
-// requests 51 -> 36 us, 2999 requests 56 -> 49 us (98 -> 53 us with sources off
+// requests 51 -> 36 us, 2999 requests 56 -> 46 us (98 -> 52 us with sources off
 // by 4 to 12 bytes).  From some 5000 requests on, reading every request in
 // every CTA costs more than a plan kernel (6000: 65 against 62 us).
 constexpr int kSmallRequests = 4096;
@@ -526,29 +526,50 @@ __global__ void __launch_bounds__(256, 3)
   // every request: its size in 16-byte units (scalar stores: the top bit)
   unsigned long long bytes = 0, chunks = 0;
   unsigned err = ~0u;
-  for (unsigned k = 0; k < per; ++k) {
-    const unsigned i = t + k * T;
-    unsigned units = 0;
-    if (i < (unsigned)n) {
-      const nvshmemx_request r = load_request(src, (int)i, compact != 0);
-      if (keep && blockIdx.x == 0) store_request(keep + i, r);
-      WorkItem w;
-      unsigned cnt;
-      const int e = plan_one(c, r, chunk, w, cnt);
-      if (e) {
-        const unsigned code = (i << 8) | (unsigned)e;
-        err = code < err ? code : err;
-      } else {
-        chunks += cnt;
-        if (w.kind == kCopy) {
-          bytes += w.len;
-          units = (unsigned)((w.len + 15ull) >> 4);
-        } else {
-          units = 1u << 31;
-        }
+  for (unsigned k0 = 0; k0 < per; k0 += 4) {
+    // four at a time: one after the other, each waits for its own load
+    uint4 lo[4], hi[4];
+#pragma unroll
+    for (unsigned j = 0; j < 4; ++j) {
+      const unsigned i = t + (k0 + j) * T;
+      if (k0 + j < per && i < (unsigned)n) {
+        const uint4 *q = reinterpret_cast<const uint4 *>(src) + (compact ? i : 2 * i);
+        lo[j] = q[0];
+        if (!compact) hi[j] = q[1];
       }
     }
-    sh.pre[t * per + k] = units;
+#pragma unroll
+    for (unsigned j = 0; j < 4; ++j) {
+      const unsigned k = k0 + j, i = t + k * T;
+      if (k >= per) break;
+      unsigned units = 0;
+      if (i < (unsigned)n) {
+        nvshmemx_request r;
+        if (compact) {
+          r = expand_compact(lo[j]);
+        } else {
+          memcpy(&r, &lo[j], 16);
+          memcpy(reinterpret_cast<char *>(&r) + 16, &hi[j], 16);
+        }
+        if (keep && blockIdx.x == 0) store_request(keep + i, r);
+        WorkItem w;
+        unsigned cnt;
+        const int e = plan_one(c, r, chunk, w, cnt);
+        if (e) {
+          const unsigned code = (i << 8) | (unsigned)e;
+          err = code < err ? code : err;
+        } else {
+          chunks += cnt;
+          if (w.kind == kCopy) {
+            bytes += w.len;
+            units = (unsigned)((w.len + 15ull) >> 4);
+          } else {
+            units = 1u << 31;
+          }
+        }
+      }
+      sh.pre[t * per + k] = units;
+    }
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
