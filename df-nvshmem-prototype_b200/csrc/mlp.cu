@@ -17,8 +17,8 @@
 // memory from step to step, the partial gradients are read by their owners
 // through distributed shared memory, and a step costs two cluster barriers
 // instead of three launches.  800 rows, batch 128: 75 us a step as a memset, a
-// gradient kernel (64 threads per 32 rows) and an Adam kernel, 12 us now, of
-// which the tile takes 5 us and the exchange of gradients and weights 6 us.
+// gradient kernel (64 threads per 32 rows) and an Adam kernel, 11 us now, half of
+// it the tile and half the exchange of gradients and weights.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <string.h>
@@ -36,6 +36,11 @@ constexpr int NI = NVSHMEMX_PICKER_NIN, NH = NVSHMEMX_PICKER_HIDDEN, NO = NVSHME
 constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + NH * NI, OFF_W2 = OFF_B1 + NH, OFF_B2 = OFF_W2 + NH * NH,
               OFF_W3 = OFF_B2 + NH, OFF_B3 = OFF_W3 + NH * NH, OFF_W4 = OFF_B3 + NH, OFF_B4 = OFF_W4 + NO * NH,
               NPARAM = OFF_B4 + NO;
+// The gradient in shared memory has the rows of W1 padded to 8, so that every
+// group of four values is one 16-byte access there and in the network.
+constexpr int NPAD = NPARAM + NH * 2;
+__host__ __device__ constexpr int padded(int p) { return p < OFF_B1 ? (p / NI) * 8 + p % NI : p + NH * 2; }
+static_assert(NPAD % 4 == 0 && padded(OFF_W2) % 4 == 0 && padded(OFF_W4) % 4 == 0, "16-byte groups");
 constexpr int kThreads = 256;
 constexpr int kRows = 16;       // rows of a tile of the grid kernels
 constexpr int kTrainRows = 8;   // rows of a CTA's tile in a training cluster
@@ -56,22 +61,23 @@ template <int R>
 struct NetGrad : Net<R> {
   float Y[R * NO], M[R * NO];
   float D1[R * LD], D2[R * LD], D3[R * LD];  // dL/dz of the hidden layers
-  float G[NPARAM + 4];                                   // gradient, in the parameters' own order
+  float G[NPAD];                             // gradient (padded order)
   float loss;
 };
 
-// Where parameter p lies in the net's shared memory, in floats from its start.
-__host__ __device__ __forceinline__ int param_slot(int p) {
+// Where the value at padded position q lies in the net's shared memory, in
+// floats from its start.
+__host__ __device__ __forceinline__ int net_slot(int q) {
   constexpr int sW2 = NH * LDX, sW3 = sW2 + NH * LD, sW4 = sW3 + NH * LD, sb1 = sW4 + NO * LD, sb2 = sb1 + NH,
                 sb3 = sb2 + NH, sb4 = sb3 + NH;
-  if (p < OFF_B1) return (p / NI) * LDX + p % NI;
-  if (p < OFF_W2) return sb1 + (p - OFF_B1);
-  if (p < OFF_B2) return sW2 + ((p - OFF_W2) / NH) * LD + (p - OFF_W2) % NH;
-  if (p < OFF_W3) return sb2 + (p - OFF_B2);
-  if (p < OFF_B3) return sW3 + ((p - OFF_W3) / NH) * LD + (p - OFF_W3) % NH;
-  if (p < OFF_W4) return sb3 + (p - OFF_B3);
-  if (p < OFF_B4) return sW4 + ((p - OFF_W4) / NH) * LD + (p - OFF_W4) % NH;
-  return sb4 + (p - OFF_B4);
+  if (q < NH * 8) return (q / 8) * LDX + q % 8;
+  if (q < padded(OFF_W2)) return sb1 + (q - padded(OFF_B1));
+  if (q < padded(OFF_B2)) return sW2 + ((q - padded(OFF_W2)) / NH) * LD + (q - padded(OFF_W2)) % NH;
+  if (q < padded(OFF_W3)) return sb2 + (q - padded(OFF_B2));
+  if (q < padded(OFF_B3)) return sW3 + ((q - padded(OFF_W3)) / NH) * LD + (q - padded(OFF_W3)) % NH;
+  if (q < padded(OFF_W4)) return sb3 + (q - padded(OFF_B3));
+  if (q < padded(OFF_B4)) return sW4 + ((q - padded(OFF_W4)) / NH) * LD + (q - padded(OFF_W4)) % NH;
+  return sb4 + (q - padded(OFF_B4));
 }
 
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
@@ -83,7 +89,7 @@ __device__ __forceinline__ void load_net(Net<R> &s, const float *__restrict__ P)
   for (int i = t; i < R * LDX; i += kThreads) s.X[i] = 0.f;
   __syncthreads();
   float *base = s.W1;
-  for (int p = t; p < NPARAM; p += kThreads) base[param_slot(p)] = P[p];
+  for (int p = t; p < NPARAM; p += kThreads) base[net_slot(padded(p))] = P[p];
 }
 
 // out[r][j] = relu(b[j] + sum_k W[j][k] in[r][k]): a warp takes 32 outputs
@@ -250,11 +256,11 @@ __device__ __forceinline__ void tile_gradient(NetGrad<R> &s, int rows, float inv
       g[2] += d * a.z;
       g[3] += d * a.w;
     }
-    put_grad4(s.G + OFF_W4 + q * NH + i4, g, first);
+    put_grad4(s.G + padded(OFF_W4) + q * NH + i4, g, first);
   } else if (t < NO * 16 + NO) {
     float g = 0.f;
     for (int r = 0; r < R; ++r) g += s.O[r * 16 + (t - NO * 16)];
-    put_grad(s.G + OFF_B4 + (t - NO * 16), g, first);
+    put_grad(s.G + padded(OFF_B4) + (t - NO * 16), g, first);
   }
   if (t < R * 16) {
     const int r = t >> 4, i4 = (t & 15) * 4;
@@ -273,10 +279,10 @@ __device__ __forceinline__ void tile_gradient(NetGrad<R> &s, int rows, float inv
         m.x > 0.f ? a[0] : 0.f, m.y > 0.f ? a[1] : 0.f, m.z > 0.f ? a[2] : 0.f, m.w > 0.f ? a[3] : 0.f);
   }
   __syncthreads();
-  weight_grad<R>(s.D3, s.A2, s.G + OFF_W3, s.G + OFF_B3, first);
+  weight_grad<R>(s.D3, s.A2, s.G + padded(OFF_W3), s.G + padded(OFF_B3), first);
   input_grad<R>(s.D3, s.W3, s.A2, s.D2);
   __syncthreads();
-  weight_grad<R>(s.D2, s.A1, s.G + OFF_W2, s.G + OFF_B2, first);
+  weight_grad<R>(s.D2, s.A1, s.G + padded(OFF_W2), s.G + padded(OFF_B2), first);
   input_grad<R>(s.D2, s.W2, s.A1, s.D1);
   __syncthreads();
   // layer 1: one output's inputs f and f + 4 per thread; the bias where
@@ -290,9 +296,9 @@ __device__ __forceinline__ void tile_gradient(NetGrad<R> &s, int rows, float inv
       if (f + 4 < NI) g1 += d * s.X[r * LDX + f + 4];
       sb += d;
     }
-    put_grad(s.G + OFF_W1 + j * NI + f, g0, first);
-    if (f + 4 < NI) put_grad(s.G + OFF_W1 + j * NI + f + 4, g1, first);
-    if (f == 3) put_grad(s.G + OFF_B1 + j, sb, first);
+    put_grad(s.G + j * 8 + f, g0, first);
+    if (f + 4 < NI) put_grad(s.G + j * 8 + f + 4, g1, first);
+    if (f == 3) put_grad(s.G + padded(OFF_B1) + j, sb, first);
   }
 }
 
@@ -357,7 +363,7 @@ __global__ void __launch_bounds__(kThreads) mlp_grad_kernel(const float *__restr
   }
   __syncthreads();
   if (first) return;
-  for (int p = t; p < NPARAM; p += kThreads) atomicAdd(&grad[p], s.G[p]);
+  for (int p = t; p < NPARAM; p += kThreads) atomicAdd(&grad[p], s.G[padded(p)]);
   if (t == 0) atomicAdd(loss, s.loss);
 }
 
@@ -377,10 +383,10 @@ struct TrainTile {
   int pad;
 };
 enum { kFirst = 1, kLast = 2 };
-constexpr int kCluster = 16;                                          // CTAs (8 took 14.4 us a step, 16 12.0 us)
+constexpr int kCluster = 16;                                          // CTAs (8 took 14.4 us a step, 16 12.0 us; 11.0 with 16-byte exchanges)
 constexpr int kTileRows = kCluster * kTrainRows;                           // rows of a tile
-constexpr int kOwned = (NPARAM + kCluster - 1) / kCluster;              // parameters a CTA updates ...
-constexpr int kPerThread = (kOwned + kThreads - 1) / kThreads;          // ... and a thread of it
+constexpr int kOwned = (NPAD / 4 + kCluster - 1) / kCluster;          // 16-byte groups that a CTA updates,
+static_assert(kOwned <= kThreads, "");                                // one of them per thread
 // A batch of more rows is spread over more SMs than a cluster has: 512 rows
 // take the cluster 39 us a step, the three launches of a spread-out step 37 us;
 // 256 rows 22 us.
@@ -396,8 +402,17 @@ __device__ __forceinline__ float ld_peer(unsigned a) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_peer(unsigned a, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+__device__ __forceinline__ float4 ld_peer4(unsigned a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(a)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_peer4(unsigned a, float4 v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+               : "memory");
 }
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release;" ::: "memory");
@@ -405,10 +420,10 @@ __device__ __forceinline__ void cluster_barrier() {
 }
 
 // Every CTA holds the whole network and takes 8 of a tile's 128 rows.  After
-// a batch's last tile, CTA c sums the cluster's gradients of parameters
+// a batch's last tile, CTA c sums the cluster's gradients of the 16-byte groups
 // [c * kOwned, (c + 1) * kOwned) in rank order (so training is reproducible),
-// updates them (their moments stay in its registers) and writes the new
-// values into every CTA's network.  The next tile's rows, and the row numbers
+// updates those parameters (their moments stay in its registers) and writes
+// the new values into every CTA's network.  The next tile's rows, and the row numbers
 // of the one after, are fetched while a tile is computed.
 __global__ void __launch_bounds__(kThreads) train_cluster_kernel(float *__restrict__ P, float *__restrict__ Am,
                                                                  float *__restrict__ Av, const float *__restrict__ X,
@@ -423,21 +438,21 @@ __global__ void __launch_bounds__(kThreads) train_cluster_kernel(float *__restri
   const int t = threadIdx.x, rank = blockIdx.x;
   load_net(s, P);
   if (t == 0) s.loss = 0.f;
-  float p[kPerThread], m[kPerThread], v[kPerThread];
+  // this thread's group of parameters: padded positions q .. q + 3, and their
+  // numbers (-1: padding, or no group)
+  const int q = (rank * kOwned + t) * 4;
+  const bool own = t < kOwned && q < NPAD;
+  float p[4], m[4], v[4];
+  int num[4];
 #pragma unroll
-  for (int i = 0; i < kPerThread; ++i) {
-    const int q = t + i * kThreads, g = rank * kOwned + q;
-    const bool own = q < kOwned && g < NPARAM;
-    p[i] = own ? P[g] : 0.f;
-    m[i] = own ? Am[g] : 0.f;
-    v[i] = own ? Av[g] : 0.f;
+  for (int i = 0; i < 4; ++i) {
+    num[i] = !own ? -1 : q < NH * 8 ? ((q + i) % 8 < NI ? (q + i) / 8 * NI + (q + i) % 8 : -1) : q + i - NH * 2;
+    p[i] = num[i] >= 0 ? P[num[i]] : 0.f;
+    m[i] = num[i] >= 0 ? Am[num[i]] : 0.f;
+    v[i] = num[i] >= 0 ? Av[num[i]] : 0.f;
   }
-  int slot[kPerThread];
-#pragma unroll
-  for (int i = 0; i < kPerThread; ++i) {
-    const int g = rank * kOwned + t + i * kThreads;
-    slot[i] = param_slot(g < NPARAM ? g : 0);
-  }
+  const float *const g_at = s.G + (own ? q : 0), *const p_at = s.W1 + net_slot(own ? q : 0);
+  if (t < NH * 2) s.G[t / 2 * 8 + NI + t % 2] = 0.f;  // the padding of W1's gradient
   // this thread's part of a tile: one output of one row, one input of one row
   const int yr = t / NO, yk = t % NO, xr = t / NI, xf = t % NI;
   const bool has_y = t < kTrainRows * NO, has_x = t < kTrainRows * NI;
@@ -484,31 +499,32 @@ __global__ void __launch_bounds__(kThreads) train_cluster_kernel(float *__restri
         epoch_loss = 0.f;
       }
     }
+    if (own) {
+      float4 part[kCluster];
 #pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-      const int q = t + k * kThreads, g = rank * kOwned + q;
-      if (q < kOwned && g < NPARAM) {
-        float part[kCluster];
+      for (unsigned r = 0; r < kCluster; ++r) part[r] = ld_peer4(peer_addr(g_at, r));
+      float g[4] = {part[0].x, part[0].y, part[0].z, part[0].w};
 #pragma unroll
-        for (unsigned r = 0; r < kCluster; ++r) part[r] = ld_peer(peer_addr(s.G + g, r));
-        float sum = part[0];
-#pragma unroll
-        for (int r = 1; r < kCluster; ++r) sum += part[r];
-        p[k] = adam_step(p[k], sum, &m[k], &v[k], lr, d.c1, d.c2);
-#pragma unroll
-        for (unsigned r = 0; r < kCluster; ++r) st_peer(peer_addr(s.W1 + slot[k], r), p[k]);
+      for (int r = 1; r < kCluster; ++r) {
+        g[0] += part[r].x;
+        g[1] += part[r].y;
+        g[2] += part[r].z;
+        g[3] += part[r].w;
       }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) p[k] = adam_step(p[k], g[k], &m[k], &v[k], lr, d.c1, d.c2);
+#pragma unroll
+      for (unsigned r = 0; r < kCluster; ++r) st_peer4(peer_addr(p_at, r), make_float4(p[0], p[1], p[2], p[3]));
     }
     cluster_barrier();  // the new weights are everywhere, nobody reads G or loss any more
     if (t == 0) s.loss = 0.f;
   }
 #pragma unroll
-  for (int i = 0; i < kPerThread; ++i) {
-    const int q = t + i * kThreads, g = rank * kOwned + q;
-    if (q < kOwned && g < NPARAM) {
-      P[g] = p[i];
-      Am[g] = m[i];
-      Av[g] = v[i];
+  for (int i = 0; i < 4; ++i) {
+    if (num[i] >= 0) {
+      P[num[i]] = p[i];
+      Am[num[i]] = m[i];
+      Av[num[i]] = v[i];
     }
   }
 }
