@@ -548,18 +548,18 @@ __global__ void __launch_bounds__(256, 3) alltoall_ring_kernel(Cfg c, A2aShare s
 // contiguous, 16-byte-rounded segment per caller unit (warp or CTA), so every
 // unit streams one range; MODE_THREAD keeps the prototype's shape, one thread
 // per message through the typed per-thread call.
-// Bounds: as many threads and CTAs per SM as its callers may ask for (kThreadMany:
-// a thread per message up to 289 PEs; two CTAs, with the ring's shared memory
-// three).
+// Bounds: as many threads and CTAs per SM as its callers may ask for: a thread
+// per message up to 289 PEs (kThreadMany), two CTAs, in the CTA-wide TMA mode
+// three.
 constexpr int kThreadMany = 4;  // MODE_THREAD for more than 33 PEs
+constexpr int kUnaligned = 5;   // MODE_BULK with buffers that are not 16-byte aligned
 
 template <int MODE>
 __global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 32 : MODE == kThreadMany ? 288 : 256,
-                                  MODE == NVSHMEMX_MODE_BULK ? 3 : 2)
+                                  MODE == kUnaligned ? 3 : 2)
     alltoall_kernel(Cfg c, int op, int dtype, unsigned long long send_off,
                                 unsigned long long recv_off, unsigned long long bytes, int rounds, int nsets,
-                                unsigned long long set_stride, unsigned bulk_smem, int device_barrier) {
-  extern __shared__ __align__(128) char smem[];
+                                unsigned long long set_stride, int device_barrier) {
   const int pe = blockIdx.z, np = c.npes;
   const unsigned long long total = (unsigned long long)(np - 1) * bytes;
   unsigned long long unit, nunits;
@@ -608,10 +608,8 @@ __global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 32 : MODE == kT
         const unsigned long long t0 = rec ? gtimer() : 0;
         if (MODE == NVSHMEMX_MODE_WARP)
           copy_coop<16, 8, 4>(dst, src, len, threadIdx.x & 31, 32);
-        else if (MODE == NVSHMEMX_MODE_BLOCK)  // one CTA per SM: 12 vectors in flight per lane (16 MiB a round 302 us, 317 with 8)
-          copy_coop<16, 12>(dst, src, len, threadIdx.x, blockDim.x);
-        else
-          bulk_copy_block(c, dst, src, len, smem, bulk_smem);
+        else  // one CTA per SM: 12 vectors in flight per lane (16 MiB a round 302 us, 317 with 8)
+          copy_coop<16, MODE == NVSHMEMX_MODE_BLOCK ? 12 : 8>(dst, src, len, threadIdx.x, blockDim.x);
         if (rec)
           trace_rec(c, op == NVSHMEMX_REQ_PUT ? NVSHMEMX_TRACE_PUT_INT : NVSHMEMX_TRACE_GET_INT,
                     op == NVSHMEMX_REQ_PUT ? src : dst, op == NVSHMEMX_REQ_PUT ? dst : src, len,
@@ -1182,7 +1180,11 @@ static int alltoall_setup(int op, int dtype, size_t send_off, size_t recv_off, s
     default: {
       // the ring that runs across rounds needs every buffer 16-byte aligned
       const bool aligned = ((bytes | send_off | recv_off | (nsets > 1 ? set_stride : 0)) & 15) == 0;
-      *fn = aligned ? (const void *)alltoall_ring_kernel : (const void *)alltoall_kernel<NVSHMEMX_MODE_BULK>;
+      // (without it the block form's copies are ahead of a TMA ring per message,
+      // which only some messages can use: 1,048,580 bytes 26.1 against 33.1 us a
+      // round, 12,000,008 bytes 235 against 301; the mode still records no puts)
+      *fn = aligned ? (const void *)alltoall_ring_kernel : (const void *)alltoall_kernel<kUnaligned>;
+      if (!aligned) *smem = 0;
     }
   }
   return 0;
@@ -1194,7 +1196,7 @@ static int alltoall_launch(const void *fn, dim3 grid, dim3 block, unsigned smem,
   Cfg c = rt().cfg;
   unsigned long long so = send, ro = recv, by = bytes, ss = stride;
   if (fn != (const void *)alltoall_ring_kernel) {
-    void *args[] = {&c, &op, &dtype, &so, &ro, &by, &rounds, &nsets, &ss, &smem, &device_barrier};
+    void *args[] = {&c, &op, &dtype, &so, &ro, &by, &rounds, &nsets, &ss, &device_barrier};
     return launch_collective(fn, grid, block, args, smem, 0);
   }
   A2aShare share = {op, 0, nsets, so, ro, ss, by, 0, 0};
