@@ -409,8 +409,9 @@ __device__ __forceinline__ void a2a_message(const Cfg &c, int op, int pe, unsign
 // round's first chunks are issued before this round's barrier, so a round no
 // longer starts by waiting for its first load (8 PEs, us a round with a ring
 // per round and now: 4 KiB messages 3.0 and 2.76, 256 KiB 8.2 and 7.2, 1 MiB
-// 21.6 and 20.9).  Every chunk stays inside one message; all addresses are 16-byte aligned (the
-// caller checks).  Stage reuse lags one store behind, as in bulk_copy_1t.
+// 21.6 and 20.9).  Every chunk stays inside one message; all addresses are
+// 16-byte aligned (the caller checks).  Stage reuse lags one store behind, as
+// in bulk_copy_1t.
 // Shared memory: 8 mbarriers, the destination and length of each stage's chunk
 // (256 bytes), then the stages.
 constexpr unsigned kA2aStages = 6;
@@ -546,8 +547,8 @@ __global__ void __launch_bounds__(256, 3) alltoall_ring_kernel(Cfg c, A2aShare s
 // Message k (0..npes-2) of PE p goes to / comes from peer q = (p+1+k) % npes.
 // For the cooperative modes the PE's (npes-1)*bytes are cut into one
 // contiguous, 16-byte-rounded segment per caller unit (warp or CTA), so every
-// unit streams one range; MODE_THREAD keeps the prototype's shape, one thread
-// per message through the typed per-thread call.
+// unit streams one range; MODE_THREAD has one thread per message, as the
+// per-thread put and get (whose copies a warp's lanes share).
 // Bounds: as many threads and CTAs per SM as its callers may ask for: a thread
 // per message up to 289 PEs (kThreadMany), two CTAs, in the CTA-wide TMA mode
 // three.

@@ -94,8 +94,8 @@ int nvshmemx_batch_execute(nvshmemx_batch *b, int reps, float *out_ms);
  * the copy precedes the plan and exec kernels on the batch's stream; from
  * 8192 requests on, the batch runs as two pieces: a second stream copies
  * and plans the first quarter (in whole 256-request blocks), then the rest,
- * while the batch's stream executes each piece once it is planned, and a
- * one-thread kernel writes the status word into pinned host memory.  An
+ * while the batch's stream executes each piece once it is planned.  An error
+ * reaches the host through a pinned word that the kernels write.  An
  * invalid request in the second piece is reported after the first piece has
  * run (with one piece, nothing runs).  In stream mode the copy precedes the
  * streaming kernel.  The requests stay resident: nvshmemx_batch_execute
