@@ -3,6 +3,7 @@
 // application of the prototype writes by hand: they call nvshmem_int_put,
 // nvshmem_int_p, nvshmem_int_wait_until, nvshmem_quiet ... from inside one
 // collective launch in which blockIdx.z is the PE.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdio.h>
 
@@ -16,6 +17,8 @@
 #include "runtime.h"
 
 namespace nvshm {
+
+namespace cg = cooperative_groups;
 
 // Grow-only device scratch owned by the library (request uploads, results).
 struct DevScratch {
@@ -109,8 +112,62 @@ __device__ __forceinline__ char *slice_ptr(const Cfg &c, int pe, unsigned long l
 // the lanes of a warp so reach the shared copy together (branching to the six
 // typed calls would split them into groups); in the other forms the copy is
 // part of the kernel, which has registers for more accesses in flight.
+//
+// In the thread form the warps of a cluster of CTAs share the long copies: one
+// warp's copy moves 20-25 GB/s, so the longest of them decided when the kernel
+// ended (25,000 calls of log-normal sizes, 282 MB moved, 110 and 132 us for two
+// seeds; 83 us for both since).  A copy of kShareFrom bytes on is listed in
+// its CTA's shared memory, and each warp, done with its shorter copies, claims
+// pieces from its CTA's list and then from the others'.  (With 32 requests to a
+// warp: 88-90 us; one CTA of 192 threads instead of four of 128 95 and 102 us,
+// two of 96 threads 89 and 94, eight of 192 95 us; pieces of half the size,
+// copies from 32 KiB on, 97-100 us, since each piece starts with loads that no
+// prefetch has covered.)
+constexpr int kShareThreads = 128, kShareCtas = 4;
+constexpr unsigned kSharePiece = 32768, kShareFrom = 65536;
+
+struct SharedCopies {
+  unsigned long long dst[kShareThreads], src[kShareThreads], bytes[kShareThreads];
+  unsigned next[kShareThreads];  // pieces of the copy claimed so far
+  unsigned count;
+};
+
+// Lists a thread's copy.
+__device__ __forceinline__ void share_copy(SharedCopies &l, char *dst, const char *src, unsigned long long bytes) {
+  const unsigned k = atomicAdd(&l.count, 1u);
+  l.dst[k] = (unsigned long long)dst;
+  l.src[k] = (unsigned long long)src;
+  l.bytes[k] = bytes;
+  l.next[k] = 0;
+}
+
+// A warp's part of the copies that the cluster's CTAs have listed.
+__device__ __forceinline__ void run_shared(SharedCopies *own, unsigned lane) {
+  const cg::cluster_group cluster = cg::this_cluster();
+  const unsigned rank = cluster.block_rank(), ctas = cluster.num_blocks();
+#pragma unroll 1
+  for (unsigned i = 0; i < ctas; ++i) {
+    SharedCopies *l = cluster.map_shared_rank(own, (rank + i) % ctas);
+    const unsigned count = l->count;
+#pragma unroll 1
+    for (unsigned k = 0; k < count; ++k) {
+      const unsigned long long bytes = l->bytes[k], dst = l->dst[k], src = l->src[k];
+#pragma unroll 1
+      for (;;) {
+        unsigned p = 0;
+        if (lane == 0) p = atomicAdd(&l->next[k], 1u);
+        const unsigned long long at = (unsigned long long)__shfl_sync(0xffffffffu, p, 0) * kSharePiece;
+        if (at >= bytes) break;
+        copy_warp<16>(reinterpret_cast<char *>(dst + at), reinterpret_cast<const char *>(src + at),
+                      bytes - at < kSharePiece ? bytes - at : kSharePiece, lane);
+      }
+    }
+  }
+}
+
 template <int MODE>
-__device__ __forceinline__ void copy_request(const Cfg &c, const nvshmemx_request &r, char *smem, unsigned bulk_smem) {
+__device__ __forceinline__ void copy_request(const Cfg &c, const nvshmemx_request &r, char *smem, unsigned bulk_smem,
+                                             SharedCopies *list = nullptr) {
   const bool put = r.op == NVSHMEMX_REQ_PUT;
   unsigned long long bytes = r.dtype == NVSHMEMX_DT_DOUBLE   ? r.bytes & ~7u
                              : r.dtype < NVSHMEMX_DT_DOUBLE ? r.bytes & ~3u
@@ -132,9 +189,17 @@ __device__ __forceinline__ void copy_request(const Cfg &c, const nvshmemx_reques
                    (MODE == NVSHMEMX_MODE_THREAD ||
                     (MODE == NVSHMEMX_MODE_WARP ? (threadIdx.x & 31) == 0 : threadIdx.x == 0));
   const unsigned long long t0 = rec ? gtimer() : 0;
-  if (MODE == NVSHMEMX_MODE_THREAD)
+  if (MODE == NVSHMEMX_MODE_THREAD) {
+    // a traced copy stays with its warp: the record times it
+    if (bytes >= kShareFrom && !c.trace) {
+      share_copy(*list, dst, src, bytes);
+      bytes = 0;
+    }
+    cg::this_cluster().sync();
     copy_lanes<16, 12, true>(dst, src, bytes);
-  else if (MODE == NVSHMEMX_MODE_WARP)
+    run_shared(list, threadIdx.x & 31);
+    cg::this_cluster().sync();  // nobody claims from this CTA's list any more
+  } else if (MODE == NVSHMEMX_MODE_WARP)
     copy_warp<12>(dst, src, bytes, threadIdx.x & 31);
   else if (MODE == NVSHMEMX_MODE_BLOCK)
     copy_coop<16, 8>(dst, src, bytes, threadIdx.x, blockDim.x);
@@ -146,11 +211,12 @@ __device__ __forceinline__ void copy_request(const Cfg &c, const nvshmemx_reques
   }
 }
 
-// CTAs of two warps in the thread and warp forms: a CTA's place frees up with
-// its longest request, and 25,000 one-thread requests still give every SM
-// work.  The warp form runs 20 warps per SM with 12 vectors in flight each:
-// 100,000 requests 255-270 us, against 300-360 us with 24 warps of 8 vectors
-// in CTAs of eight (its largest request, one warp's, is a third of that time).
+// CTAs of two warps in the warp form: a CTA's place frees up with its longest
+// request.  It runs 20 warps per SM with 12 vectors in flight each: 100,000
+// requests 255-270 us, against 300-360 us with 24 warps of 8 vectors in CTAs of
+// eight (its largest request, one warp's, is a third of that time).  Sharing
+// the long copies as in the thread form, in CTAs of two to eight warps, took
+// 278-299 us where this takes 257: a warp then waits for its CTA's others.
 //
 // The CTA forms have two shapes.  A CTA spends about 2 us on a short request
 // (its descriptor, then its data), so many requests want many CTAs: 128 threads,
@@ -163,30 +229,32 @@ __device__ __forceinline__ void copy_request(const Cfg &c, const nvshmemx_reques
 constexpr int kManyBlock = 6144, kManyBulk = 12288;
 
 template <int MODE, int THREADS>
-__global__ void __launch_bounds__(THREADS, MODE == NVSHMEMX_MODE_THREAD ? 6
+__global__ void __launch_bounds__(THREADS, MODE == NVSHMEMX_MODE_THREAD ? 384 / THREADS
                                            : MODE == NVSHMEMX_MODE_WARP ? 10
                                            : THREADS == 128             ? 7
                                                                         : 3)
-    exec_requests_kernel(Cfg c, const nvshmemx_request *__restrict__ reqs, int n, unsigned bulk_smem) {
+    exec_requests_kernel(Cfg c, const nvshmemx_request *__restrict__ reqs, int n, unsigned bulk_smem,
+                         unsigned lanes) {
   extern __shared__ __align__(128) char smem[];
   long long u;
   if (MODE == NVSHMEMX_MODE_THREAD)
-    u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    // `lanes` of a warp have a request (see launch_exec_requests)
+    u = (threadIdx.x & 31) < lanes
+            ? (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes + (threadIdx.x & 31)
+            : n;
   else if (MODE == NVSHMEMX_MODE_WARP)
     u = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   else
     u = blockIdx.x;
   nvshmemx_request r;
   if (MODE == NVSHMEMX_MODE_THREAD) {
-    // every lane takes part in the warp's copies, those without one too
+    // every thread takes part in the copies, those without a request too
     r.op = 0xff;
     r.bytes = 0;
     r.dtype = 0;
     r.src_pe = r.dst_pe = 0;
     r.src_off = r.dst_off = 0;
     if (u < n) r = reqs[u];
-    copy_request<MODE>(c, r, smem, bulk_smem);
-    if (u >= n || r.op <= NVSHMEMX_REQ_GET) return;
   } else {
     if (u >= n) return;
     r = reqs[u];
@@ -197,7 +265,7 @@ __global__ void __launch_bounds__(THREADS, MODE == NVSHMEMX_MODE_THREAD ? 6
   switch (r.op) {
     case NVSHMEMX_REQ_PUT:
     case NVSHMEMX_REQ_GET:
-      copy_request<MODE>(c, r, smem, bulk_smem);
+      if (MODE != NVSHMEMX_MODE_THREAD) copy_request<MODE>(c, r, smem, bulk_smem);
       break;
     case NVSHMEMX_REQ_SIGNAL:
       if (leader) nvshmemx_int_signal((int *)(c.arena + r.dst_off), r.value, r.dst_pe);
@@ -223,7 +291,14 @@ __global__ void __launch_bounds__(THREADS, MODE == NVSHMEMX_MODE_THREAD ? 6
       }
       break;
     default:
-      if (leader) record_error(c, NVSHMEMX_ERR_INVALID, (long long)u);
+      if (leader && u < n) record_error(c, NVSHMEMX_ERR_INVALID, (long long)u);
+  }
+  if (MODE == NVSHMEMX_MODE_THREAD) {
+    // last: the request's other fields need no registers during the copies
+    __shared__ SharedCopies list;
+    if (threadIdx.x == 0) list.count = 0;
+    __syncthreads();
+    copy_request<MODE>(c, r, smem, bulk_smem, &list);
   }
 }
 
@@ -955,24 +1030,44 @@ int launch_exec_requests(int mode, const nvshmemx_request *dr, int n, cudaStream
   const Cfg c = rt().cfg;
   if (n <= 0) return 0;
   switch (mode) {
-    case NVSHMEMX_MODE_THREAD:
-      exec_requests_kernel<NVSHMEMX_MODE_THREAD, 64><<<(n + 63) / 64, 64, 0, s>>>(c, dr, n, 0);
+    case NVSHMEMX_MODE_THREAD: {
+      // Requests to a warp: no more than keep the warps of two CTAs to an SM
+      // busy (up to 38,000 requests; 4100 of median 16 KiB took 322 us with 32
+      // to a warp in CTAs of 64 threads, 110 so; 600 of 64 KiB 527 and 76 us;
+      // 1000 of 2 KiB 47 and 30; for one CTA to an SM 116, 96 and 30 us).
+      const long long warps = (long long)rt().sm_count * (2 * kShareThreads / 32);
+      const unsigned lanes = (unsigned)std::min<long long>(32, (n + warps - 1) / warps);
+      const long long per = (long long)lanes * (kShareThreads / 32) * kShareCtas;
+      cudaLaunchAttribute at = {};
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = kShareCtas;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cudaLaunchConfig_t lc = {};
+      lc.gridDim = dim3((unsigned)((n + per - 1) / per) * kShareCtas);
+      lc.blockDim = dim3(kShareThreads);
+      lc.stream = s;
+      lc.attrs = &at;
+      lc.numAttrs = 1;
+      const cudaError_t e =
+          cudaLaunchKernelEx(&lc, exec_requests_kernel<NVSHMEMX_MODE_THREAD, kShareThreads>, c, dr, n, 0u, lanes);
+      if (e != cudaSuccess) return check_cuda(e, "exec_requests launch");
       break;
+    }
     case NVSHMEMX_MODE_WARP:
-      exec_requests_kernel<NVSHMEMX_MODE_WARP, 64><<<(n + 1) / 2, 64, 0, s>>>(c, dr, n, 0);
+      exec_requests_kernel<NVSHMEMX_MODE_WARP, 64><<<(n + 1) / 2, 64, 0, s>>>(c, dr, n, 0, 0);
       break;
     case NVSHMEMX_MODE_BLOCK:
       if (n > kManyBlock)
-        exec_requests_kernel<NVSHMEMX_MODE_BLOCK, 128><<<n, 128, 0, s>>>(c, dr, n, 0);
+        exec_requests_kernel<NVSHMEMX_MODE_BLOCK, 128><<<n, 128, 0, s>>>(c, dr, n, 0, 0);
       else
-        exec_requests_kernel<NVSHMEMX_MODE_BLOCK, 256><<<n, 256, 0, s>>>(c, dr, n, 0);
+        exec_requests_kernel<NVSHMEMX_MODE_BLOCK, 256><<<n, 256, 0, s>>>(c, dr, n, 0, 0);
       break;
     default: {
       const bool many = n > kManyBulk;
       const auto fn = many ? exec_requests_kernel<NVSHMEMX_MODE_BULK, 128> : exec_requests_kernel<NVSHMEMX_MODE_BULK, 256>;
       const unsigned smem = many ? kBulkSmemMany : kBulkSmem;
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      fn<<<n, many ? 128 : 256, smem, s>>>(c, dr, n, smem);
+      fn<<<n, many ? 128 : 256, smem, s>>>(c, dr, n, smem, 0);
     }
   }
   return check_cuda(cudaGetLastError(), "exec_requests launch");
