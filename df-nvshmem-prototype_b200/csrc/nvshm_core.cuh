@@ -529,19 +529,26 @@ __device__ __forceinline__ void copy_own(char *dst, const char *src, unsigned nv
 // 2 KiB, up to 3 MiB, 282 MB moved) took 1240-2060 us with every lane on its
 // own, as long as the longest call takes one thread; together 115-140 us.
 // A lane whose copy has at most kOwn vectors, or operands that are not 4-byte
-// aligned, copies it itself, as do fewer than kTogether lanes.  LU / SU: the
-// vectors in flight per lane for long and short copies.  FULL: the caller
-// knows that all 32 lanes are here.
+// aligned, copies it itself, as do fewer than kTogether lanes, and a lane with
+// an operand in its own local memory, where the same address names another
+// array in every other lane.  LU / SU: the vectors in flight per lane for long
+// and short copies.  FULL: the caller knows that all 32 lanes are here, with
+// operands in the heap.
 //
 // The first __syncwarp makes what a lane wrote before its call visible to the
 // lanes that copy for it, the last one makes their stores the calling lane's
 // (its later fences and signals order them like its own).
 template <int LU, int SU, bool FULL = false>
 __device__ __forceinline__ void copy_lanes(char *dst, const char *src, unsigned long long bytes) {
-  const unsigned mask = FULL ? 0xffffffffu : __activemask();
+  unsigned mask = 0xffffffffu;
+  bool local = false;
+  if (!FULL) {
+    local = __isLocal(dst) || __isLocal(src);
+    mask = __ballot_sync(__activemask(), !local);
+  }
   const unsigned nl = FULL ? 32u : __popc(mask);
   const unsigned mis = (unsigned)((uintptr_t)dst ^ (uintptr_t)src);
-  if (!FULL && nl < kTogether) {
+  if (!FULL && (local || nl < kTogether)) {
     // one thread: 16 vector accesses in flight (measured 2.6x the bandwidth of
     // 4 for a 1 MiB put) and an L2 prefetch 64 rounds (16 KiB) ahead: 1 MiB
     // from DRAM 0.90 -> 1.36 GB/s, from L2 1.89 -> 1.81 GB/s
