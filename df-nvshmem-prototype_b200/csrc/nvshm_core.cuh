@@ -172,6 +172,8 @@ template <> struct VecT<1> { typedef unsigned char T; };
 
 // Asks the TMA unit to stage [p, p + bytes) in L2 (16-byte aligned address,
 // size a multiple of 16; nothing to wait for -- later loads just hit L2).
+// Only for addresses in global memory: callers ask __isGlobal of a source that
+// an application named.
 __device__ __forceinline__ void l2_prefetch_bulk(uintptr_t p, unsigned bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes));
 }
@@ -269,7 +271,7 @@ __device__ __forceinline__ void copy_body(char *__restrict__ dst, const char *__
   unsigned long long i = r;
   const unsigned long long step = (unsigned long long)nthr * U;
   const unsigned long long dist = (unsigned long long)PFI * step * VB;  // bytes ahead
-  const bool pf_on = PFI > 0 && r == 0 && nthr <= 32 && bytes >= 2 * dist;
+  const bool pf_on = PFI > 0 && r == 0 && nthr <= 32 && bytes >= 2 * dist && __isGlobal(src);
   const uintptr_t pf_end = ((uintptr_t)src + bytes) & ~(uintptr_t)15;
   uintptr_t pf = ((uintptr_t)src + 15) & ~(uintptr_t)15;  // next source byte to stage
   if (nv >= (unsigned long long)(U - 1) * nthr) {
@@ -325,7 +327,7 @@ __device__ __forceinline__ void copy_tiles(char *__restrict__ dst, const char *_
   const unsigned nw = n >> 5, w = r >> 5, lane = r & 31u;
   // operands a number of bytes apart: in rows of four only (load_row)
   const unsigned long long ntiles = (mis & 3) == 0 ? nv / (U * 32) : 0;
-  const bool pf_on = PFI > 0 && n == 32 && lane == 0 && ntiles >= 2ull * PFI;
+  const bool pf_on = PFI > 0 && n == 32 && lane == 0 && ntiles >= 2ull * PFI && __isGlobal(src);
   const uintptr_t pf_end = ((uintptr_t)src + nv * 16) & ~(uintptr_t)15;
   uintptr_t pf = ((uintptr_t)src + 15) & ~(uintptr_t)15;  // next source byte to stage
   const char *s = src + (unsigned long long)w * TB + lane * 16u;
@@ -424,6 +426,7 @@ template <int U>
 __device__ __forceinline__ unsigned copy_warp_long(unsigned lane, char *dst, const char *src, unsigned nv,
                                                    unsigned mis) {
   const unsigned rounds = nv / (U * 32);
+  const bool pf_on = lane == 0 && __isGlobal(src);
   const uintptr_t pf_end = ((uintptr_t)src + (unsigned long long)nv * 16u) & ~(uintptr_t)15;
   uintptr_t pf = ((uintptr_t)src + 15) & ~(uintptr_t)15;
   const char *s = src + 16u * lane;
@@ -432,7 +435,7 @@ __device__ __forceinline__ unsigned copy_warp_long(unsigned lane, char *dst, con
   for (unsigned k = 0; k < rounds; ++k) {
     uint4 v[U];
     load_row<U>(v, s, mis, U);
-    if (lane == 0) {
+    if (pf_on) {
       uintptr_t want = ((uintptr_t)s + kAhead) & ~(uintptr_t)15;
       if (want > pf_end) want = pf_end;
       if (want >= pf + 4096) {
@@ -748,8 +751,8 @@ __device__ __forceinline__ bool bulk_copy_1t(const BulkRing &ring, char *dst, co
 
 // Block-cooperative bulk copy: thread 0 drives the TMA ring over the
 // 16-aligned body while the other threads copy the unaligned head and tail.
-// Falls back to the generic copy when dst/src alignments differ mod 16 or the
-// ring has no room.  Every thread of the block must call it.
+// Falls back to the generic copy when dst/src alignments differ mod 16, an
+// operand is not in global memory or the ring has no room.  Every thread of the block must call it.
 // One issuer per CTA streams the body as one sequential range: measured on
 // B200 this keeps DRAM accesses more local than splitting the range across
 // per-warp rings (which lost 6-7% on 16-256 MiB all-to-all rounds).
@@ -759,7 +762,7 @@ __device__ __forceinline__ void bulk_copy_block(const Cfg &c, char *dst, const c
   const unsigned r = block_rank(), n = block_size();
   BulkRing ring = make_ring(smem, smem_bytes, 6);
   if ((((uintptr_t)dst ^ (uintptr_t)src) & 15) != 0 || ring.stage_bytes < 1024 || bytes < 4096 ||
-      n < 64) {
+      n < 64 || !__isGlobal(dst) || !__isGlobal(src)) {
     copy_coop<16, 4>(dst, src, bytes, r, n);
     __syncthreads();
     return;

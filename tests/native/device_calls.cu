@@ -9,9 +9,10 @@
 // list.  The lists run one after the other.
 //
 // Forms: 0 one thread per request, the lanes of the mask in every warp; 1 warp,
-// 2 CTA, 3 CTA through the TMA ring.  Operand (form 0): where the local side of
-// a put or get lies: 0 the heap, 1 an array of the thread's own, 2 shared memory
-// (a part for each thread), 3 shared memory (one source for all threads).
+// 2 CTA, 3 CTA through the TMA ring.  Operand: where the local side of a put or
+// get lies: 0 the heap, 1 an array of the thread's own, 2 shared memory (a part
+// for each thread), 3 shared memory (one source for all requests); forms 1 to 3
+// take 0 and 3.
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -25,7 +26,7 @@
 
 static const int kWords = 68;        // of a thread's own array
 static const int kSource = 24 << 10;  // bytes of the source for all threads
-static const int kRing = 32 << 10;
+static const int kRing = 20 << 10;
 
 __device__ void call(const nvshmemx_request &r, void *sym, void *near, bool put) {
   const int pe = put ? r.dst_pe : r.src_pe;
@@ -45,16 +46,19 @@ __device__ void copy_words(int *dst, const int *src, unsigned bytes) {
   for (unsigned i = 0; i < bytes / 4; ++i) dst[i] = src[i];
 }
 
+// The first request's source in shared memory, by all threads.
+__device__ void load_source(char *shared, char *arena, const nvshmemx_request &r) {
+  const char *src = (const char *)nvshmemx_ptr(arena + r.src_off, r.src_pe);
+  for (unsigned i = threadIdx.x; i < r.bytes; i += blockDim.x) shared[i] = src[i];
+  __syncthreads();
+}
+
 __global__ void by_thread(char *arena, const nvshmemx_request *reqs, int n, unsigned lanes, int operand) {
   __shared__ __align__(16) char shared[kSource];
   __align__(16) int own[kWords];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const int k = (int)(blockIdx.x * (blockDim.x >> 5) + warp) * __popc(lanes) + __popc(lanes & ((1u << lane) - 1u));
-  if (operand == 3) {
-    const char *src = (const char *)nvshmemx_ptr(arena + reqs[0].src_off, reqs[0].src_pe);
-    for (unsigned i = threadIdx.x; i < reqs[0].bytes; i += blockDim.x) shared[i] = src[i];
-    __syncthreads();
-  }
+  if (operand == 3) load_source(shared, arena, reqs[0]);
   if ((lanes >> lane & 1u) && k < n) {
     const nvshmemx_request r = reqs[k];
     const bool put = r.op == NVSHMEMX_REQ_PUT;
@@ -75,14 +79,16 @@ __global__ void by_thread(char *arena, const nvshmemx_request *reqs, int n, unsi
   __syncwarp();
 }
 
-__global__ void by_group(char *arena, const nvshmemx_request *reqs, int n, int form) {
+__global__ void by_group(char *arena, const nvshmemx_request *reqs, int n, int form, int operand) {
   extern __shared__ __align__(128) char ring[];
+  __shared__ __align__(16) char shared[kSource];
+  if (operand == 3) load_source(shared, arena, reqs[0]);
   const int k = form == 1 ? (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) : (int)blockIdx.x;
   if (k >= n) return;
   const nvshmemx_request r = reqs[k];
   const bool put = r.op == NVSHMEMX_REQ_PUT;
   char *sym = arena + (put ? r.dst_off : r.src_off);
-  void *near = nvshmemx_ptr(arena + (put ? r.src_off : r.dst_off), put ? r.src_pe : r.dst_pe);
+  void *near = operand == 3 ? shared : nvshmemx_ptr(arena + (put ? r.src_off : r.dst_off), put ? r.src_pe : r.dst_pe);
   const int pe = put ? r.dst_pe : r.src_pe;
   if (form == 3) {
     if (put) nvshmemx_putmem_bulk_block(sym, near, r.bytes, pe, ring, kRing);
@@ -143,7 +149,7 @@ int main(int argc, char **argv) {
       const int per = __builtin_popcount((unsigned)s[1]) * 2;  // of a CTA of two warps
       by_thread<<<(s[2] + per - 1) / per, 64>>>(arena, d, s[2], (unsigned)s[1], s[3]);
     } else {
-      by_group<<<s[0] == 1 ? (s[2] + 3) / 4 : s[2], 128, s[0] == 3 ? kRing : 0>>>(arena, d, s[2], s[0]);
+      by_group<<<s[0] == 1 ? (s[2] + 3) / 4 : s[2], 128, s[0] == 3 ? kRing : 0>>>(arena, d, s[2], s[0], s[3]);
     }
     CHECK(cudaGetLastError());
     CHECK(cudaDeviceSynchronize());

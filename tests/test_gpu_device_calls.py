@@ -99,10 +99,14 @@ def test_local_operand_of_the_thread(exe, tmp_path, operand):
 
 
 def test_long_copies_from_shared_memory(exe, tmp_path):
-    """From 16 KiB on a copy prefetches its source, which only memory can be."""
+    """From 16 KiB on a copy prefetches its source, and the TMA form loads it
+    into its ring: both only from global memory."""
     m = Rows()
-    check(exe, tmp_path, [(0, lanes, SHARED_ONE, m.make([nb], bin(lanes).count("1"), op=REQ_PUT, same_source=True))
-                          for lanes in (0x100, 0x7FFF, ALL) for nb in (16384, 20484, 24576)])
+    lists = [(0, lanes, SHARED_ONE, m.make([nb], bin(lanes).count("1"), op=REQ_PUT, same_source=True))
+             for lanes in (0x100, 0x7FFF, ALL) for nb in (16384, 20484, 24576)]
+    lists += [(form, ALL, SHARED_ONE, m.make([nb], 5, op=REQ_PUT, same_source=True))
+              for form in (1, 2, 3) for nb in (4100, 24576)]
+    check(exe, tmp_path, lists)
 
 
 @pytest.mark.parametrize("dtype", [DT_INT, DT_FLOAT, DT_DOUBLE])
