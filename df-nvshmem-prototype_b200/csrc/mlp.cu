@@ -586,10 +586,10 @@ struct nvshmemx_mlp {
   int cluster = -1;  // whether a training cluster fits the device (-1: not asked yet)
   int dev = 0, slot = -1;
   // Device copies of the host arrays of a call, kept between calls up to
-  // kKeep bytes; a larger call allocates its own.  `mu` holds a call's use of
-  // them (and of G and loss), so calls on one network from several threads
-  // run one after the other.
-  std::mutex mu;
+  // kKeep bytes; a larger call allocates its own.  `mu` is held for the whole of
+  // every call but destroy, so calls on one network from several threads run
+  // one after the other.
+  mutable std::mutex mu;
   char *work = nullptr;
   size_t work_bytes = 0;
   bool work_own = false;  // allocated (else part of a slot)
@@ -748,7 +748,13 @@ int nvshmemx_mlp_destroy(nvshmemx_mlp *m) {
   if (!m) return 0;
   if (m->work_own) cudaFree(m->work);
   if (m->slot >= 0) {
-    cudaStreamSynchronize(0);  // nothing of this network runs any more (a free would wait too)
+    // nothing of this network runs any more (a free would wait too): the wait
+    // is for the network's device, whichever is current
+    int now = m->dev;
+    cudaGetDevice(&now);
+    if (now != m->dev) cudaSetDevice(m->dev);
+    cudaStreamSynchronize(0);
+    if (now != m->dev) cudaSetDevice(now);
     give_slot(m->dev, m->slot);
   } else if (m->block) {
     cudaFree(m->block);
@@ -759,11 +765,13 @@ int nvshmemx_mlp_destroy(nvshmemx_mlp *m) {
 
 int nvshmemx_mlp_get_params(const nvshmemx_mlp *m, float *h) {
   if (!m || !h) return fail(NVSHMEMX_ERR_INVALID, "mlp_get_params");
+  std::lock_guard<std::mutex> lk(m->mu);
   return check_cuda(cudaMemcpy(h, m->P, NPARAM * 4, cudaMemcpyDeviceToHost), "mlp_get_params");
 }
 
 int nvshmemx_mlp_set_params(nvshmemx_mlp *m, const float *h) {
   if (!m || !h) return fail(NVSHMEMX_ERR_INVALID, "mlp_set_params");
+  std::lock_guard<std::mutex> lk(m->mu);
   return check_cuda(cudaMemcpy(m->P, h, NPARAM * 4, cudaMemcpyHostToDevice), "mlp_set_params");
 }
 
@@ -774,6 +782,7 @@ int nvshmemx_mlp_set_normalization(nvshmemx_mlp *m, const float *mean, const flo
     h[i] = mean[i];
     h[NI + i] = sd[i] > 1e-12f ? sd[i] : 1.f;
   }
+  std::lock_guard<std::mutex> lk(m->mu);
   return check_cuda(cudaMemcpy(m->norm, h, sizeof h, cudaMemcpyHostToDevice), "mlp_set_normalization");
 }
 
@@ -816,6 +825,7 @@ int nvshmemx_mlp_train(nvshmemx_mlp *m, const float *X, const float *Y, const fl
   std::vector<double> rowm(n, 0.0);
   for (int i = 0; i < n; ++i)
     for (int k = 0; k < NO; ++k) rowm[i] += M[(size_t)i * NO + k];
+  Work w(m);
   const bool one_cluster = batch <= kClusterBatch && cluster_fits(m);
   const int nb = (n - 1) / batch + 1;  // batches of an epoch
   // epochs to a launch: at most 4 MiB of row numbers
@@ -824,7 +834,6 @@ int nvshmemx_mlp_train(nvshmemx_mlp *m, const float *X, const float *Y, const fl
   // one block: features, targets, masks, row numbers, tiles, losses
   const size_t xb = pad256((size_t)n * NI * 4), yb = pad256((size_t)n * NO * 4), ib = pad256((size_t)per * n * 4),
                tb = one_cluster ? pad256(per * tiles_epoch * sizeof(TrainTile)) : 0, lb = pad256((size_t)epochs * 4);
-  Work w(m);
   int rc;
   if ((rc = w.get(m, xb + 2 * yb + ib + tb + lb))) return rc;
   float *dX = (float *)w.p, *dY = (float *)(w.p + xb), *dM = (float *)(w.p + xb + yb);
