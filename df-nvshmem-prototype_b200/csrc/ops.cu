@@ -378,14 +378,18 @@ __global__ void checksum_kernel(const unsigned long long *p, unsigned long long 
 // the kernel with the checks and the trace record of nvshmem_int_put: the call
 // would save and restore the registers of its group copy (exchanges of
 // 4, 68 and 1020 bytes 3.35, 3.71 and 8.5 us with the call, 2.94, 3.05 and 7.7
-// without).
+// without).  Whole vectors go straight to the copy: the branches around the
+// words outside them cost a short exchange more than those words (16, 64 and
+// 256 bytes 2.29, 2.28 and 2.38 us an exchange through them, 2.20, 2.20 and
+// 2.27 straight).
 __device__ __forceinline__ void put_ints_alone(const Cfg &c, int *target, const int *source, int len, int pe) {
   const unsigned long long bytes = elem_bytes<int>(len);
   if (!check_remote(c, target, bytes, pe) || !check_local(c, source, bytes)) return;
   char *dst = xlate(c, target, pe);
   const unsigned long long t0 = c.trace ? gtimer() : 0;
   const char *src = reinterpret_cast<const char *>(source);
-  if ((((uintptr_t)dst | (uintptr_t)src) & 3) != 0) {
+  const uintptr_t at = (uintptr_t)dst | (uintptr_t)src;
+  if ((at & 3) != 0 || ((at | bytes) & 15) == 0) {
     copy_coop<16, 16, 64>(dst, src, bytes, 0, 1);
   } else {
     // the words outside the destination's vectors, loaded before those
@@ -410,6 +414,9 @@ __device__ __forceinline__ void put_ints_alone(const Cfg &c, int *target, const 
   if (c.trace) trace_rec(c, NVSHMEMX_TRACE_PUT_INT, source, dst, bytes, pe, t0, gtimer());
 }
 
+// DATA: a payload goes before the flag.  Without one the kernel is a flag's
+// round trip alone, in 26 registers instead of 220 (760 -> 704 ns).
+template <bool DATA>
 __global__ void pingpong_kernel(Cfg c, int *data, int *flag, int len, int iters, int skip, long long *cycles,
                                 unsigned long long *gt) {
   const int pe = nvshmemx_my_pe();
@@ -421,7 +428,7 @@ __global__ void pingpong_kernel(Cfg c, int *data, int *flag, int len, int iters,
     if (i == skip) g0 = nvshm::gtimer();
     long long t = clock64();
     if (pe == 0) {
-      if (len > 0) {
+      if (DATA) {
         put_ints_alone(c, data, my_data, len, 1);
         nvshmem_quiet();
       }
@@ -429,7 +436,7 @@ __global__ void pingpong_kernel(Cfg c, int *data, int *flag, int len, int iters,
       nvshmem_int_wait(my_flag, i);
     } else {
       nvshmem_int_wait(my_flag, i);
-      if (len > 0) {
+      if (DATA) {
         put_ints_alone(c, data, my_data, len, 0);
         nvshmem_quiet();
       }
@@ -1170,7 +1177,8 @@ int nvshmemx_op_pingpong(size_t flag_off, size_t data_off, int len_elems, int it
       return rc;
   Cfg c = r.cfg;
   void *args[] = {&c, &data, &flag, &len_elems, &iters, &skip, &cyc, &gt};
-  if ((rc = launch_collective((const void *)pingpong_kernel, dim3(1), dim3(32), args, 0, 0))) return rc;
+  const void *fn = len_elems > 0 ? (const void *)pingpong_kernel<true> : (const void *)pingpong_kernel<false>;
+  if ((rc = launch_collective(fn, dim3(1), dim3(32), args, 0, 0))) return rc;
   if ((rc = check_cuda(cudaDeviceSynchronize(), "pingpong"))) return rc;
   std::vector<long long> h(iters);
   unsigned long long total = 0;
