@@ -276,7 +276,14 @@ __device__ __forceinline__ WorkItem load_item(const WorkItem *p) {
   return w;
 }
 
-template <int VB, int U>
+// TIGHT: the register-copy kernel, which has 64 registers a thread (its CTAs
+// may have 1024) and keeps the next item in them.  The engine of copy_coop
+// spilled there (456 bytes with U = 8, in the aligned loop too: 25,000 requests
+// 73 -> 96 us, 100,000 240 -> 293 us), so operands off by less than a vector
+// take copy_body with as many whole vectors in flight as fit: the aligned loop
+// is back at 72 us (60,000 requests: 140 -> 189 -> 138 us), and sources off by
+// 4 to 12 bytes take 77 us (narrow accesses both ways 91, copy_coop 90 us).
+template <int VB, int U, bool TIGHT = false>
 __device__ __forceinline__ void run_item(const WorkItem &w, unsigned lane) {
   if (w.kind == kCopy) {
     char *d = reinterpret_cast<char *>(w.dst);
@@ -284,14 +291,21 @@ __device__ __forceinline__ void run_item(const WorkItem &w, unsigned lane) {
     // copies off by less than a vector go to the engine that stores whole
     // vectors all the same (copy_coop); the common case keeps its own short
     // loop (25,000 requests: 90.3 us a pass with it, 91.0 us without)
-    if (VB == 16 && (((uintptr_t)d ^ (uintptr_t)s) & 15) == 0)
+    if (VB == 16 && (mis & 15) == 0)
+    const unsigned mis = (unsigned)((uintptr_t)d ^ (uintptr_t)s);
       copy_body<16, U>(d, s, w.len, lane, 32);
-    else
+    else if (!TIGHT || VB < 16)
       copy_coop<VB, U>(d, s, w.len, lane, 32);
   } else if (lane == 0) {
     // Requests of one batch are unordered with respect to each other (they
     // touch disjoint bytes), so a SIGNAL is a plain 4-byte store like
     // nvshmem_int_p; completion of the batch orders it before later work.
+    else if ((mis & 3) != 0)
+      copy_body<1, 4>(d, s, w.len, lane, 32);
+    else if ((mis & 7) != 0)
+      copy_body<16, U == 8 ? 4 : U == 4 ? 3 : 2, 0, 4>(d, s, w.len, lane, 32);
+    else
+      copy_body<16, U >= 4 ? 4 : 2, 0, 8>(d, s, w.len, lane, 32);
     if (w.kind == kSignal) {
       st_relaxed_b32(reinterpret_cast<void *>(w.dst), (unsigned)w.value);
     } else if (w.len == 8) {
@@ -324,7 +338,7 @@ __global__ void __launch_bounds__(1024) batch_exec_kernel(const WorkItem *__rest
     for (unsigned long long k = base; k < end; ++k) {
       WorkItem nx;
       if (k + 1 < end) nx = load_item(items + k + 1);
-      run_item<VB, U>(cur, lane);
+      run_item<VB, U, true>(cur, lane);
       cur = nx;
     }
     base = __shfl_sync(0xffffffffu, nxt, 0);
