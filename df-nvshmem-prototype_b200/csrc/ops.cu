@@ -632,13 +632,13 @@ __global__ void __launch_bounds__(256, 3) alltoall_ring_kernel(Cfg c, A2aShare s
 // unit streams one range; MODE_THREAD has one thread per message, as the
 // per-thread put and get (whose copies a warp's lanes share).
 // Bounds: as many threads and CTAs per SM as its callers may ask for: a thread
-// per message up to 289 PEs (kThreadMany), two CTAs, in the CTA-wide TMA mode
-// three.
-constexpr int kThreadMany = 4;  // MODE_THREAD for more than 33 PEs
+// per message up to 129 PEs and (kThreadMany) up to 289, two CTAs, in the
+// CTA-wide TMA mode three.
+constexpr int kThreadMany = 4;  // MODE_THREAD for more than 129 PEs
 constexpr int kUnaligned = 5;   // MODE_BULK with buffers that are not 16-byte aligned
 
 template <int MODE>
-__global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 32 : MODE == kThreadMany ? 288 : 256,
+__global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 128 : MODE == kThreadMany ? 288 : 256,
                                   MODE == kUnaligned ? 3 : 2)
     alltoall_kernel(Cfg c, int op, int dtype, unsigned long long send_off,
                                 unsigned long long recv_off, unsigned long long bytes, int rounds, int nsets,
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 32 : MODE == kT
       if (mine) a2a_message(c, op, pe, so, ro, bytes, unit, &dst, &src);
       const bool rec = mine && c.trace;
       const unsigned long long t0 = rec ? gtimer() : 0;
-      copy_lanes<8, MODE == NVSHMEMX_MODE_THREAD ? 8 : 4, true>(dst, src, mine ? bytes : 0);
+      copy_lanes<MODE == NVSHMEMX_MODE_THREAD ? 8 : 4, MODE == NVSHMEMX_MODE_THREAD ? 8 : 2, true>(dst, src, mine ? bytes : 0);
       if (rec)
         trace_rec(c, (op == NVSHMEMX_REQ_PUT ? NVSHMEMX_TRACE_PUT_INT : NVSHMEMX_TRACE_GET_INT) + dtype,
                   op == NVSHMEMX_REQ_PUT ? src : dst, op == NVSHMEMX_REQ_PUT ? dst : src, bytes,
@@ -1270,11 +1270,12 @@ static int alltoall_setup(int op, int dtype, size_t send_off, size_t recv_off, s
   *block = dim3(256);
   switch (mode) {
     case NVSHMEMX_MODE_THREAD:
-      // one warp holds the messages of up to 33 PEs: its kernel has the
-      // registers for 8 vectors in flight per lane (7 messages of 4 KiB 4.8 us a
-      // round, 11 us with the 4 of the kernel for more PEs, 7.9 us with every
-      // message copied by one lane)
-      *fn = r.npes <= 33 ? (const void *)alltoall_kernel<NVSHMEMX_MODE_THREAD>
+      // CTAs of up to 128 threads have the registers for 8 vectors in flight per
+      // lane, larger ones for 4 and 2 (with more they spill).  Us a round with 4096
+      // bytes to a message, with each lane on its own, with 4 in flight, and now:
+      // 34 PEs 25.6, 44.5, 16.4; 64 PEs 52.7, 90.7, 26.9; 128 PEs 105, 115, 37.6;
+      // (4 and 2) 160 PEs 183, 123, 90; 200 PEs 324, 136, 98
+      *fn = r.npes <= 129 ? (const void *)alltoall_kernel<NVSHMEMX_MODE_THREAD>
                          : (const void *)alltoall_kernel<kThreadMany>;
       *grid = dim3(1);
       *block = dim3(32 * ((r.npes - 1 + 31) / 32));
