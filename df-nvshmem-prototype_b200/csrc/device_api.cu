@@ -52,7 +52,7 @@ __device__ __noinline__ void putmem_coop(void *target, const void *source, unsig
   // 16 MiB block / warp all-to-all 0.66 / 0.72 -> 0.81 / 0.91 of the copy peak);
   // a warp also prefetches into L2 4 rounds (16 KiB) ahead: 1 MiB from DRAM
   // 13.3 -> 20.6 GB/s, from L2 28.7 -> 27.1 GB/s; C4 calls 3133 -> 3601 GB/s
-  nvshm::copy_coop<16, 8, 4>(dst, reinterpret_cast<const char *>(source), bytes, r, n);
+  nvshm::copy_coop<16, 8, 4, true>(dst, reinterpret_cast<const char *>(source), bytes, r, n);
   if (c.trace && r == 0) nvshm::trace_rec(c, op, source, dst, bytes, pe, t0, nvshm::gtimer());
 }
 
@@ -62,7 +62,7 @@ __device__ __noinline__ void getmem_coop(void *target, const void *source, unsig
   if (!nvshm::check_remote(c, source, bytes, pe) || !nvshm::check_local(c, target, bytes)) return;
   const char *src = nvshm::xlate(c, source, pe);
   unsigned long long t0 = (c.trace && r == 0) ? nvshm::gtimer() : 0;
-  nvshm::copy_coop<16, 8, 4>(reinterpret_cast<char *>(target), src, bytes, r, n);
+  nvshm::copy_coop<16, 8, 4, true>(reinterpret_cast<char *>(target), src, bytes, r, n);
   if (c.trace && r == 0) nvshm::trace_rec(c, op, target, src, bytes, pe, t0, nvshm::gtimer());
 }
 

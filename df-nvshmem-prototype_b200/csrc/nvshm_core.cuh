@@ -320,7 +320,16 @@ __device__ __forceinline__ void copy_body(char *__restrict__ dst, const char *__
 // vectors (a stride known only at run time costs an address pair for each of
 // the U accesses both ways: 72 instead of 60 registers for U = 8).
 // PFI > 0: a lone warp keeps an L2 prefetch PFI tiles ahead (see copy_body).
-template <int U, unsigned PFI>
+//
+// Tiles go in whole rounds of the block's warps; what is left would occupy some
+// of them only (a message of 16 KiB is three of the all-to-all's tiles: 64 PEs
+// 53 us a round by strides of the block, 68 with a tile to a warp, 45 so) and
+// goes in rows.  EVEN deals the rows out over all warps, for a CTA that has its
+// SM to itself (messages of 4100 bytes 48 -> 41 us a round); without it a warp
+// takes four at a time, so that short copies occupy few warps where many CTAs
+// share an SM (100,000 puts and gets of median 2 KiB, a CTA each: 272 us, 285
+// with the rows dealt out).
+template <int U, unsigned PFI, bool EVEN>
 __device__ __forceinline__ void copy_tiles(char *__restrict__ dst, const char *__restrict__ src,
                                            unsigned long long nv, unsigned mis, unsigned r, unsigned n) {
   constexpr unsigned TB = U * 512;  // bytes per tile
@@ -332,9 +341,10 @@ __device__ __forceinline__ void copy_tiles(char *__restrict__ dst, const char *_
   uintptr_t pf = ((uintptr_t)src + 15) & ~(uintptr_t)15;  // next source byte to stage
   const char *s = src + (unsigned long long)w * TB + lane * 16u;
   char *d = dst + (unsigned long long)w * TB + lane * 16u;
+  unsigned long long done = 0;  // tiles, in whole rounds of the warps
   if (w < nw) {
 #pragma unroll 1
-    for (unsigned long long t = w; t < ntiles; t += nw) {
+    for (; done + nw <= ntiles; done += nw) {
       uint4 v[U];
       load_row<U>(v, s, mis, U);
       if (pf_on) {
@@ -352,17 +362,17 @@ __device__ __forceinline__ void copy_tiles(char *__restrict__ dst, const char *_
       d += (unsigned long long)nw * TB;
     }
   }
-  // the vectors after the last whole tile: rounds of 4 rows of 32 for a warp,
-  // the same rows dealt out over the warps of a block
-  const unsigned long long left = nv - ntiles * (U * 32);
-  s = src + ntiles * TB + 16u * lane;
-  d = dst + ntiles * TB + 16u * lane;
+  // the vectors after the last round of tiles: up to 4 rows of 32 at a time
+  const unsigned long long left = nv - done * (U * 32);
+  s = src + done * TB + 16u * lane;
+  d = dst + done * TB + 16u * lane;
+  const unsigned q = !EVEN || left > nw * 96 ? 128 : left > nw * 64 ? 96 : left > nw * 32 ? 64 : 32;
   if (w < nw) {
 #pragma unroll 1
-    for (unsigned long long i = w * 128; i < left; i += nw * 128) {
+    for (unsigned long long i = w * q; i < left; i += nw * q) {
       uint4 v[4];
-      const unsigned rows = left - i < 128 ? (unsigned)(left - i) : 128u;  // vectors of this round
-      const unsigned have = rows > lane ? (rows - lane + 31) / 32 : 0;     // this lane's
+      const unsigned rows = left - i < q ? (unsigned)(left - i) : q;    // vectors of this round
+      const unsigned have = rows > lane ? (rows - lane + 31) / 32 : 0;  // this lane's
       load_row<4>(v, s + i * 16, mis, have);
 #pragma unroll
       for (unsigned u = 0; u < 4; ++u)
@@ -374,7 +384,8 @@ __device__ __forceinline__ void copy_tiles(char *__restrict__ dst, const char *_
 // One thread, one warp or a block copies `bytes`: 16-byte stores, with loads
 // as wide as the relative alignment of dst and src allows.  MAXV caps the
 // width of both (4 and 8: the batch engine's narrow configurations).
-template <int MAXV = 16, int U = 4, unsigned PFI = 0>
+// EVEN: see copy_tiles.
+template <int MAXV = 16, int U = 4, unsigned PFI = 0, bool EVEN = false>
 __device__ __forceinline__ void copy_coop(char *dst, const char *src, unsigned long long bytes,
                                           unsigned r, unsigned nthr) {
   const unsigned mis = (unsigned)((uintptr_t)dst ^ (uintptr_t)src);
@@ -410,7 +421,7 @@ __device__ __forceinline__ void copy_coop(char *dst, const char *src, unsigned l
   }
   dst += head;
   src += head;
-  copy_tiles<U, PFI>(dst, src, nv, mis, r, nthr);
+  copy_tiles<U, PFI, EVEN>(dst, src, nv, mis, r, nthr);
 }
 
 // ----------------------------------------------- one copy per thread, shared

@@ -692,7 +692,7 @@ __global__ void __launch_bounds__(MODE == NVSHMEMX_MODE_THREAD ? 128 : MODE == k
         if (MODE == NVSHMEMX_MODE_WARP)
           copy_coop<16, 8, 4>(dst, src, len, threadIdx.x & 31, 32);
         else  // one CTA per SM: 12 vectors in flight per lane (16 MiB a round 302 us, 317 with 8)
-          copy_coop<16, MODE == NVSHMEMX_MODE_BLOCK ? 12 : 8>(dst, src, len, threadIdx.x, blockDim.x);
+          copy_coop<16, MODE == NVSHMEMX_MODE_BLOCK ? 12 : 8, 0, true>(dst, src, len, threadIdx.x, blockDim.x);
         if (rec)
           trace_rec(c, op == NVSHMEMX_REQ_PUT ? NVSHMEMX_TRACE_PUT_INT : NVSHMEMX_TRACE_GET_INT,
                     op == NVSHMEMX_REQ_PUT ? src : dst, op == NVSHMEMX_REQ_PUT ? dst : src, len,
