@@ -169,9 +169,9 @@ template <int MODE>
 __device__ __forceinline__ void copy_request(const Cfg &c, const nvshmemx_request &r, char *smem, unsigned bulk_smem,
                                              SharedCopies *list = nullptr) {
   const bool put = r.op == NVSHMEMX_REQ_PUT;
-  unsigned long long bytes = r.dtype == NVSHMEMX_DT_DOUBLE   ? r.bytes & ~7u
-                             : r.dtype < NVSHMEMX_DT_DOUBLE ? r.bytes & ~3u
-                                                            : (r.bytes >> 2) * 8ull;
+  unsigned long long bytes = r.dtype == NVSHMEMX_DT_DOUBLE                                  ? r.bytes & ~7u
+                             : r.dtype < NVSHMEMX_DT_DOUBLE || MODE == NVSHMEMX_MODE_BULK ? r.bytes & ~3u
+                                                                                           : (r.bytes >> 2) * 8ull;
   char *near = slice_ptr(c, put ? r.src_pe : r.dst_pe, put ? r.src_off : r.dst_off);
   const char *sym = c.arena + (put ? r.dst_off : r.src_off);
   const int pe = put ? r.dst_pe : r.src_pe;
