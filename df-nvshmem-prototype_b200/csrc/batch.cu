@@ -481,21 +481,28 @@ __global__ void __launch_bounds__(256, 3) batch_exec_tma_kernel(const WorkItem *
 }
 
 // ------------------------------------------------ small batches: one launch
-// Below kSmallRequests requests, planning is done by every CTA for itself: it
-// reads all requests (at most 128 KB, from L2 or, for a few, from the kernel's
-// parameters), checks them, and builds the running count of pieces in its own
-// shared memory.  No CTA waits for another and nothing has to be zeroed, so
-// the memset, the plan kernel and the exec kernel become one launch; an
-// invalid request is seen by every CTA, and none copies anything.  Pieces are
-// a power of two of bytes, at most the configured chunk and about two for
-// each warp of the grid, so a batch of few requests still spreads over every
-// SM (with 16 KiB chunks a 64-request batch keeps some 80 of 1184 warps
-// busy).  CTA b takes pieces b, b + gridDim.x, ..., its warps the next one
-// each.  Measured per call from pinned memory: 64 requests 49 -> 29 us, 1000
-// requests 51 -> 36 us, 2999 requests 56 -> 46 us (98 -> 52 us with sources off
-// by 4 to 12 bytes).  From some 5000 requests on, reading every request in
-// every CTA costs more than a plan kernel (6000: 65 against 62 us).
-constexpr int kSmallRequests = 4096;
+// Below kSmallPerThread requests for each thread of a CTA, planning is done by
+// every CTA for itself: it reads all requests (at most 112 KB, from L2 or, for a
+// few, from the kernel's parameters), checks them, and builds the running count
+// of pieces in its own shared memory.  No CTA waits for another and nothing has
+// to be zeroed, so the memset, the plan kernel and the exec kernel become one
+// launch; an invalid request is seen by every CTA, and none copies anything.
+// Pieces are a power of two of bytes, at most the configured chunk and about two
+// for each warp of the grid, so a batch of few requests still spreads over every
+// SM (with 16 KiB chunks a 64-request batch keeps some 80 of 1184 warps busy).
+// CTA b takes pieces b, b + gridDim.x, ..., its warps the next one each.
+//
+// What it costs is the requests that each thread reads, so that is what limits
+// it.  Times of a call as one launch and as plan and exec (submit from pinned
+// memory; execute), median request 2 KiB:
+//   CTAs of 256 threads, 3 x 8 KiB rings  1000 requests 33, 44; 26, 30 us
+//                                         3000 41, 46; 32, 32   3500 44, 46; 34, 34
+//                                         4095 47, 46; 36, 34
+//   CTAs of 128 threads, 2 x 8 KiB rings  1500 38, 46; 30, 32   2000 40, 46; 33, 33
+//                                         2500 45, 46; 36, 34   4095 53, 48; 42, 35
+// With 2 x 16 KiB rings the lines cross at 1500 and 2200 requests, with rings of
+// 1 to 4 KiB stages at 2500 to 3500.
+constexpr int kSmallPerThread = 14;
 constexpr int kParamWords = 240;  // 16-byte words of requests that fit the kernel's parameters
 
 template <int NP>
@@ -1164,7 +1171,7 @@ static const size_t kMaxSmem = 227u << 10;
 // room for the running count (the default's do, up to the limit).
 static bool small_batch(const nvshmemx_batch *b, int n) {
   const nvshmemx_batch_config &k = b->cfg;
-  return n > 0 && n < kSmallRequests && k.stream == 0 && k.tma_stages > 0 && small_smem_bytes(k, n) <= kMaxSmem;
+  return n > 0 && n < kSmallPerThread * k.threads && k.stream == 0 && k.tma_stages > 0 && small_smem_bytes(k, n) <= kMaxSmem;
 }
 
 // Enqueues a small batch on the batch's stream: n requests in device memory at

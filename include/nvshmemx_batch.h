@@ -87,10 +87,11 @@ int nvshmemx_batch_execute(nvshmemx_batch *b, int reps, float *out_ms);
 /* End-to-end call: copies n requests from host memory (pinned if it is the
  * batch's host buffer), executes them and reads back the batch status word;
  * *out_status receives the status (0 = every request done), *out_ms the
- * device time of the whole sequence.  Below 4096 requests a TMA
- * configuration runs the batch as one launch (no plan kernel, no graph; the
- * work unit is then at most chunk_bytes), and some hundred requests travel as
- * the kernel's parameters.  Otherwise, with a graph configuration (stream 0),
+ * device time of the whole sequence.  Below 14 requests to a
+ * thread of a CTA (3584 with the default 256 threads) a TMA configuration runs
+ * the batch as one launch (no plan kernel, no graph; the work unit is then at
+ * most chunk_bytes), and some hundred requests travel as the kernel's
+ * parameters.  Otherwise, with a graph configuration (stream 0),
  * the copy precedes the plan and exec kernels on the batch's stream; from
  * 8192 requests on, the batch runs as two pieces: a second stream copies
  * and plans the first quarter (in whole 256-request blocks), then the rest,
