@@ -288,24 +288,24 @@ __device__ __forceinline__ void run_item(const WorkItem &w, unsigned lane) {
   if (w.kind == kCopy) {
     char *d = reinterpret_cast<char *>(w.dst);
     const char *s = reinterpret_cast<const char *>(w.src);
+    const unsigned mis = (unsigned)((uintptr_t)d ^ (uintptr_t)s);
     // copies off by less than a vector go to the engine that stores whole
     // vectors all the same (copy_coop); the common case keeps its own short
     // loop (25,000 requests: 90.3 us a pass with it, 91.0 us without)
     if (VB == 16 && (mis & 15) == 0)
-    const unsigned mis = (unsigned)((uintptr_t)d ^ (uintptr_t)s);
       copy_body<16, U>(d, s, w.len, lane, 32);
     else if (!TIGHT || VB < 16)
       copy_coop<VB, U>(d, s, w.len, lane, 32);
-  } else if (lane == 0) {
-    // Requests of one batch are unordered with respect to each other (they
-    // touch disjoint bytes), so a SIGNAL is a plain 4-byte store like
-    // nvshmem_int_p; completion of the batch orders it before later work.
     else if ((mis & 3) != 0)
       copy_body<1, 4>(d, s, w.len, lane, 32);
     else if ((mis & 7) != 0)
       copy_body<16, U == 8 ? 4 : U == 4 ? 3 : 2, 0, 4>(d, s, w.len, lane, 32);
     else
       copy_body<16, U >= 4 ? 4 : 2, 0, 8>(d, s, w.len, lane, 32);
+  } else if (lane == 0) {
+    // Requests of one batch are unordered with respect to each other (they
+    // touch disjoint bytes), so a SIGNAL is a plain 4-byte store like
+    // nvshmem_int_p; completion of the batch orders it before later work.
     if (w.kind == kSignal) {
       st_relaxed_b32(reinterpret_cast<void *>(w.dst), (unsigned)w.value);
     } else if (w.len == 8) {
