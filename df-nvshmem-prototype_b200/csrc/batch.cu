@@ -1,6 +1,9 @@
 // batch.cu -- batched one-sided traffic (nvshmemx_batch.h).
 //
-// A batch runs as a CUDA graph of three nodes on the batch's own stream:
+// A batch of some thousand requests, with a TMA configuration, is one launch that
+// plans and executes (batch_small_kernel).  A larger one runs as a CUDA graph of
+// three nodes on the batch's own stream, a large submit as two such pieces
+// (submit_two), a streaming configuration as one cooperative launch:
 //   memset   zero the 32-byte control block (chunk count, cursor, status)
 //   plan     one thread per request: validate, translate to arena addresses,
 //            cut into chunks of <= chunk_bytes; a CTA-wide scan plus one
@@ -9,7 +12,8 @@
 //   exec     persistent grid (SM count x CTAs per SM); each warp claims
 //            `grab` chunks per atomicAdd on the cursor, prefetches the next
 //            claim and the next 32-byte work item while it copies the current
-//            chunk with VB-byte accesses, U in flight per lane.
+//            chunk with VB-byte accesses, U in flight per lane, or through a
+//            ring of shared-memory stages by TMA (batch_exec_tma_kernel).
 // Every chunk is a contiguous copy, so the exec kernel is pure streaming:
 // its roofline is HBM copy bandwidth (2 bytes moved per payload byte).
 #include <cuda_runtime.h>
@@ -320,7 +324,6 @@ template <int VB, int U>
 __global__ void __launch_bounds__(1024) batch_exec_kernel(const WorkItem *__restrict__ items, BatchCtl *ctl,
                                                           BatchCtl *sctl, unsigned long long cap, int grab) {
   const unsigned lane = threadIdx.x & 31u;
-  pdl_release_dependents();
   pdl_wait_prerequisites();
   if (!piece_may_run(ctl, sctl)) return;
   unsigned long long C = *(volatile unsigned long long *)&ctl->total_chunks;
@@ -461,7 +464,6 @@ __global__ void __launch_bounds__(256, 3) batch_exec_tma_kernel(const WorkItem *
   const unsigned lane = threadIdx.x & 31u;
   WarpTma<S> ring;
   ring.init(smem, SB, min_bulk, timeout_ns, lane);  // overlaps the plan kernel
-  pdl_release_dependents();
   pdl_wait_prerequisites();
   unsigned long long C = *(volatile unsigned long long *)&ctl->total_chunks;
   const unsigned long long ib = *(volatile unsigned long long *)&ctl->item_base;

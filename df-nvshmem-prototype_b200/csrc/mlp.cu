@@ -387,9 +387,10 @@ constexpr int kCluster = 16;                                          // CTAs (8
 constexpr int kTileRows = kCluster * kTrainRows;                           // rows of a tile
 constexpr int kOwned = (NPAD / 4 + kCluster - 1) / kCluster;          // 16-byte groups that a CTA updates,
 static_assert(kOwned <= kThreads, "");                                // one of them per thread
-// A batch of more rows is spread over more SMs than a cluster has: 512 rows
-// take the cluster 39 us a step, the three launches of a spread-out step 37 us;
-// 256 rows 22 us.
+// A batch of more rows is spread over more SMs than a cluster has.  Us a step in
+// the cluster and as three spread-out launches: 256 rows 17.7 and 32.9, 384 24.1
+// and 33.6, 512 30.6 and 34.0; 640 rows are another tile of some 6 us for the
+// cluster, and 34.8 spread out.
 constexpr int kClusterBatch = 512;
 
 __device__ __forceinline__ unsigned peer_addr(const void *p, unsigned rank) {
