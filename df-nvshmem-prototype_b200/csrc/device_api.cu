@@ -41,28 +41,29 @@ __device__ __noinline__ void get_thread(T *target, const T *source, int len, int
 }
 
 // Cooperative forms: `r` of `n` threads; bounds are checked by every thread
-// (same arguments, same answer) so all skip together.
+// (same arguments, same answer) so all skip together.  U and V: see copy_group.
+
+template <int U, int V>
 __device__ __noinline__ void putmem_coop(void *target, const void *source, unsigned long long bytes,
-                                            int pe, unsigned r, unsigned n, int op) {
+                                         int pe, unsigned r, unsigned n, int op) {
   const Cfg &c = CFG;
   if (!nvshm::check_remote(c, target, bytes, pe) || !nvshm::check_local(c, source, bytes)) return;
   char *dst = nvshm::xlate(c, target, pe);
   unsigned long long t0 = (c.trace && r == 0) ? nvshm::gtimer() : 0;
-  // 8 vector accesses in flight per thread (measured against 4 and 16: C2
-  // 16 MiB block / warp all-to-all 0.66 / 0.72 -> 0.81 / 0.91 of the copy peak);
   // a warp also prefetches into L2 4 rounds (16 KiB) ahead: 1 MiB from DRAM
-  // 13.3 -> 20.6 GB/s, from L2 28.7 -> 27.1 GB/s; C4 calls 3133 -> 3601 GB/s
-  nvshm::copy_coop<16, 8, 4, true>(dst, reinterpret_cast<const char *>(source), bytes, r, n);
+  // 13.3 -> 20.6 GB/s, from L2 28.7 -> 27.1 GB/s
+  nvshm::copy_group<U, V, 4>(dst, reinterpret_cast<const char *>(source), bytes, r, n);
   if (c.trace && r == 0) nvshm::trace_rec(c, op, source, dst, bytes, pe, t0, nvshm::gtimer());
 }
 
+template <int U, int V>
 __device__ __noinline__ void getmem_coop(void *target, const void *source, unsigned long long bytes,
-                                            int pe, unsigned r, unsigned n, int op) {
+                                         int pe, unsigned r, unsigned n, int op) {
   const Cfg &c = CFG;
   if (!nvshm::check_remote(c, source, bytes, pe) || !nvshm::check_local(c, target, bytes)) return;
   const char *src = nvshm::xlate(c, source, pe);
   unsigned long long t0 = (c.trace && r == 0) ? nvshm::gtimer() : 0;
-  nvshm::copy_coop<16, 8, 4, true>(reinterpret_cast<char *>(target), src, bytes, r, n);
+  nvshm::copy_group<U, V, 4>(reinterpret_cast<char *>(target), src, bytes, r, n);
   if (c.trace && r == 0) nvshm::trace_rec(c, op, target, src, bytes, pe, t0, nvshm::gtimer());
 }
 
@@ -205,31 +206,31 @@ __device__ void *nvshmemx_ptr(const void *sym, int pe) {
 __device__ void *nvshmemx_local_ptr(const void *sym) { return nvshmemx_ptr(sym, nvshm::my_pe(CFG)); }
 
 __device__ void nvshmemx_putmem_warp(void *target, const void *source, size_t bytes, int pe) {
-  putmem_coop(target, source, bytes, pe, lane_id(), 32, NVSHMEMX_TRACE_PUT_INT);
+  putmem_coop<8, 7>(target, source, bytes, pe, lane_id(), 32, NVSHMEMX_TRACE_PUT_INT);
 }
 __device__ void nvshmemx_getmem_warp(void *target, const void *source, size_t bytes, int pe) {
-  getmem_coop(target, source, bytes, pe, lane_id(), 32, NVSHMEMX_TRACE_GET_INT);
+  getmem_coop<8, 7>(target, source, bytes, pe, lane_id(), 32, NVSHMEMX_TRACE_GET_INT);
 }
 __device__ void nvshmemx_putmem_block(void *target, const void *source, size_t bytes, int pe) {
-  putmem_coop(target, source, bytes, pe, nvshm::block_rank(), nvshm::block_size(), NVSHMEMX_TRACE_PUT_INT);
+  putmem_coop<7, 6>(target, source, bytes, pe, nvshm::block_rank(), nvshm::block_size(), NVSHMEMX_TRACE_PUT_INT);
 }
 __device__ void nvshmemx_getmem_block(void *target, const void *source, size_t bytes, int pe) {
-  getmem_coop(target, source, bytes, pe, nvshm::block_rank(), nvshm::block_size(), NVSHMEMX_TRACE_GET_INT);
+  getmem_coop<7, 6>(target, source, bytes, pe, nvshm::block_rank(), nvshm::block_size(), NVSHMEMX_TRACE_GET_INT);
 }
 
 #define NVSHM_TYPED_COOP(Name, Type, OPP, OPG)                                                 \
   __device__ void nvshmemx_##Name##_put_warp(Type *t, Type *s, int len, int pe) {             \
-    putmem_coop(t, s, nvshm::elem_bytes<Type>(len), pe, lane_id(), 32, OPP);                  \
+    putmem_coop<8, 7>(t, s, nvshm::elem_bytes<Type>(len), pe, lane_id(), 32, OPP);                  \
   }                                                                                           \
   __device__ void nvshmemx_##Name##_get_warp(Type *t, Type *s, int len, int pe) {             \
-    getmem_coop(t, s, nvshm::elem_bytes<Type>(len), pe, lane_id(), 32, OPG);                  \
+    getmem_coop<8, 7>(t, s, nvshm::elem_bytes<Type>(len), pe, lane_id(), 32, OPG);                  \
   }                                                                                           \
   __device__ void nvshmemx_##Name##_put_block(Type *t, Type *s, int len, int pe) {            \
-    putmem_coop(t, s, nvshm::elem_bytes<Type>(len), pe, nvshm::block_rank(), nvshm::block_size(), \
+    putmem_coop<7, 6>(t, s, nvshm::elem_bytes<Type>(len), pe, nvshm::block_rank(), nvshm::block_size(), \
                 OPP);                                                                         \
   }                                                                                           \
   __device__ void nvshmemx_##Name##_get_block(Type *t, Type *s, int len, int pe) {            \
-    getmem_coop(t, s, nvshm::elem_bytes<Type>(len), pe, nvshm::block_rank(), nvshm::block_size(), \
+    getmem_coop<7, 6>(t, s, nvshm::elem_bytes<Type>(len), pe, nvshm::block_rank(), nvshm::block_size(), \
                 OPG);                                                                         \
   }
 

@@ -334,51 +334,65 @@ __device__ __forceinline__ void copy_tiles(char *__restrict__ dst, const char *_
                                            unsigned long long nv, unsigned mis, unsigned r, unsigned n) {
   constexpr unsigned TB = U * 512;  // bytes per tile
   const unsigned nw = n >> 5, w = r >> 5, lane = r & 31u;
+  if (w >= nw) return;
+  const char *s = src + w * TB + lane * 16u;
+  char *d = dst + w * TB + lane * 16u;
+  long long left = (long long)nv;  // vectors from the round's (then the row's) first on
+  const bool pf_on = PFI > 0 && n == 32 && lane == 0 && nv >= 2ull * PFI * U * 32 && __isGlobal(src);
+  int staged = 16;  // bytes from s on that are on their way to L2
   // operands a number of bytes apart: in rows of four only (load_row)
-  const unsigned long long ntiles = (mis & 3) == 0 ? nv / (U * 32) : 0;
-  const bool pf_on = PFI > 0 && n == 32 && lane == 0 && ntiles >= 2ull * PFI && __isGlobal(src);
-  const uintptr_t pf_end = ((uintptr_t)src + nv * 16) & ~(uintptr_t)15;
-  uintptr_t pf = ((uintptr_t)src + 15) & ~(uintptr_t)15;  // next source byte to stage
-  const char *s = src + (unsigned long long)w * TB + lane * 16u;
-  char *d = dst + (unsigned long long)w * TB + lane * 16u;
-  unsigned long long done = 0;  // tiles, in whole rounds of the warps
-  if (w < nw) {
+  if ((mis & 3) == 0) {
 #pragma unroll 1
-    for (; done + nw <= ntiles; done += nw) {
+    for (; left >= (long long)(nw * (U * 32)); left -= nw * (U * 32)) {
       uint4 v[U];
       load_row<U>(v, s, mis, U);
       if (pf_on) {
-        uintptr_t want = ((uintptr_t)s + PFI * TB) & ~(uintptr_t)15;
-        if (want > pf_end) want = pf_end;
-        if (want >= pf + 4096 || (want == pf_end && want > pf)) {
-          const unsigned k = (unsigned)(want - pf < 65536 ? want - pf : 65536);
-          l2_prefetch_bulk(pf, k);
-          pf += k;
+        int k = (int)(PFI * TB) - staged;
+        if (left < (long long)(PFI * U * 32)) k = (int)left * 16 - 16 - staged;
+        if (k >= 4096) {
+          l2_prefetch_bulk(((uintptr_t)s & ~(uintptr_t)15) + staged, k);
+          staged += k;
         }
+        staged -= TB;
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) *reinterpret_cast<uint4 *>(d + u * 512) = v[u];
-      s += (unsigned long long)nw * TB;
-      d += (unsigned long long)nw * TB;
+      s += nw * TB;
+      d += nw * TB;
     }
   }
   // the vectors after the last round of tiles: up to 4 rows of 32 at a time
-  const unsigned long long left = nv - done * (U * 32);
-  s = src + done * TB + 16u * lane;
-  d = dst + done * TB + 16u * lane;
   const unsigned q = !EVEN || left > nw * 96 ? 128 : left > nw * 64 ? 96 : left > nw * 32 ? 64 : 32;
-  if (w < nw) {
+  s += (int)(w * q * 16) - (int)(w * TB);
+  d += (int)(w * q * 16) - (int)(w * TB);
+  left -= w * q;
 #pragma unroll 1
-    for (unsigned long long i = w * q; i < left; i += nw * q) {
-      uint4 v[4];
-      const unsigned rows = left - i < q ? (unsigned)(left - i) : q;    // vectors of this round
-      const unsigned have = rows > lane ? (rows - lane + 31) / 32 : 0;  // this lane's
-      load_row<4>(v, s + i * 16, mis, have);
+  for (; left > 0; left -= nw * q) {
+    uint4 v[4];
+    const unsigned rows = left < q ? (unsigned)left : q;              // vectors of this round
+    const unsigned have = rows > lane ? (rows - lane + 31) / 32 : 0;  // this lane's
+    load_row<4>(v, s, mis, have);
 #pragma unroll
-      for (unsigned u = 0; u < 4; ++u)
-        if (u < have) *reinterpret_cast<uint4 *>(d + i * 16 + u * 512) = v[u];
-    }
+    for (unsigned u = 0; u < 4; ++u)
+      if (u < have) *reinterpret_cast<uint4 *>(d + u * 512) = v[u];
+    s += nw * q * 16;
+    d += nw * q * 16;
   }
+}
+
+// The bytes before and after the 16-byte vectors of the destination: fewer than
+// 32, one each for the threads r of a warp or block.  Returns how many come
+// before.
+__device__ __forceinline__ unsigned copy_edges(char *dst, const char *src, unsigned long long bytes, unsigned r) {
+  unsigned head = (unsigned)(16 - ((uintptr_t)dst & 15)) & 15u;
+  if (head > bytes) head = (unsigned)bytes;
+  const unsigned tail = (unsigned)(bytes - head) & 15u;
+  if (r < head) dst[r] = src[r];
+  if (r >= 16 && r - 16 < tail) {
+    const unsigned long long j = bytes - tail + (r - 16);
+    dst[j] = src[j];
+  }
+  return head;
 }
 
 // One thread, one warp or a block copies `bytes`: 16-byte stores, with loads
@@ -409,19 +423,35 @@ __device__ __forceinline__ void copy_coop(char *dst, const char *src, unsigned l
       copy_body<16, U, PFI, 4>(dst, src, bytes, r, nthr);
     return;
   }
-  unsigned head = (unsigned)(16 - ((uintptr_t)dst & 15)) & 15u;
-  if (head > bytes) head = (unsigned)bytes;
-  const unsigned long long nv = (bytes - head) >> 4;
-  const unsigned tail = (unsigned)(bytes - head) & 15u;
-  // fewer than 32 edge bytes: one each
-  if (r < head) dst[r] = src[r];
-  if (r >= 16 && r - 16 < tail) {
-    const unsigned long long j = bytes - tail + (r - 16);
-    dst[j] = src[j];
+  const unsigned head = copy_edges(dst, src, bytes, r);
+  copy_tiles<U, PFI, EVEN>(dst + head, src + head, (bytes - head) >> 4, mis, r, nthr);
+}
+
+// One warp or a block copies `bytes` for the public calls, whose registers are
+// those of an application's kernel, so they decide how many threads it may have
+// and how many of its CTAs run at once: at most 64 for a kernel that does little
+// else (with copy_coop such a kernel had 86 to 94 and did not run with 1024
+// threads; 592 CTAs of 256 threads took two waves).  U vectors in flight where the
+// operands are equal modulo 16, V where the loads are narrower.
+template <int U, int V, unsigned PFI>
+__device__ __forceinline__ void copy_group(char *dst, const char *src, unsigned long long bytes, unsigned r,
+                                           unsigned n) {
+  const unsigned mis = (unsigned)((uintptr_t)dst ^ (uintptr_t)src);
+  if (n < 32) {
+    if ((mis & 3) != 0)
+      copy_body<1, 4>(dst, src, bytes, r, n);
+    else if ((mis & 15) == 0)
+      copy_body<16, 4>(dst, src, bytes, r, n);
+    else
+      copy_body<4, 4>(dst, src, bytes, r, n);
+    return;
   }
-  dst += head;
-  src += head;
-  copy_tiles<U, PFI, EVEN>(dst, src, nv, mis, r, nthr);
+  const unsigned head = copy_edges(dst, src, bytes, r);
+  const unsigned long long nv = (bytes - head) >> 4;
+  if ((mis & 15) == 0)
+    copy_tiles<U, PFI, true>(dst + head, src + head, nv, 0, r, n);
+  else
+    copy_tiles<V, PFI, true>(dst + head, src + head, nv, mis, r, n);
 }
 
 // ----------------------------------------------- one copy per thread, shared
