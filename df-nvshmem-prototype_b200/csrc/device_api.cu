@@ -25,7 +25,7 @@ __device__ __noinline__ void put_thread(T *target, const T *source, int len, int
   if (!nvshm::check_remote(c, target, bytes, pe) || !nvshm::check_local(c, source, bytes)) return;
   char *dst = nvshm::xlate(c, target, pe);
   unsigned long long t0 = c.trace ? nvshm::gtimer() : 0;
-  nvshm::copy_lanes<8, 8>(dst, reinterpret_cast<const char *>(source), bytes);
+  nvshm::copy_lanes<8, 8, false, 8>(dst, reinterpret_cast<const char *>(source), bytes);
   if (c.trace) nvshm::trace_rec(c, op, source, dst, bytes, pe, t0, nvshm::gtimer());
 }
 
@@ -36,7 +36,7 @@ __device__ __noinline__ void get_thread(T *target, const T *source, int len, int
   if (!nvshm::check_remote(c, source, bytes, pe) || !nvshm::check_local(c, target, bytes)) return;
   const char *src = nvshm::xlate(c, source, pe);
   unsigned long long t0 = c.trace ? nvshm::gtimer() : 0;
-  nvshm::copy_lanes<8, 8>(reinterpret_cast<char *>(target), src, bytes);
+  nvshm::copy_lanes<8, 8, false, 8>(reinterpret_cast<char *>(target), src, bytes);
   if (c.trace) nvshm::trace_rec(c, op, target, src, bytes, pe, t0, nvshm::gtimer());
 }
 

@@ -532,11 +532,10 @@ __device__ __forceinline__ void copy_lanes_body(unsigned mask, unsigned todo, un
   }
 }
 
-// kOwn: a lane copies up to this many vectors itself (one round trip, in
-// parallel with the other lanes); kLong: from this many on (16 KiB) a copy is
-// a long one; kTogether: fewer lanes than this copy alone (together they
-// would have less in flight than each with 16 accesses of its own).
-constexpr unsigned kOwn = 4, kLong = 1024, kTogether = 16;
+// kLong: from this many vectors on (16 KiB) a copy is a long one; kTogether:
+// fewer lanes than this copy alone (together they would have less in flight than
+// each with 16 accesses of its own).
+constexpr unsigned kLong = 1024, kTogether = 16;
 
 // One copy by a warp, its long part with U vectors in flight per lane.
 template <int U>
@@ -554,15 +553,37 @@ __device__ __forceinline__ void copy_warp(char *dst, const char *src, unsigned l
   copy_coop<16, 8>(dst, src, bytes, lane, 32);
 }
 
-template <int LB>
+template <int LB, unsigned N>
 __device__ __forceinline__ void copy_own(char *dst, const char *src, unsigned nv) {
-  uint4 v[kOwn];
+  uint4 v[N];
 #pragma unroll
-  for (unsigned k = 0; k < kOwn; ++k)
+  for (unsigned k = 0; k < N; ++k)
     if (k < nv) v[k] = load16<LB>(src + 16 * k);
 #pragma unroll
-  for (unsigned k = 0; k < kOwn; ++k)
+  for (unsigned k = 0; k < N; ++k)
     if (k < nv) reinterpret_cast<uint4 *>(dst)[k] = v[k];
+}
+
+// Whether the lanes of `mask` (nl of them, with copies of `bytes` bytes between
+// operands `mis` apart) are sooner done each on its own, 16 accesses in flight,
+// than together, SU * 32.  With less than two
+// warps to an SM latency decides, not the memory's bandwidth, and copies of about
+// one length are sooner done so (a round of lanes on their own takes half as
+// long again as one together); with more warps only short ones are.  Us a launch,
+// 32 lanes of every warp together and on their own: one warp to an SM, 260 bytes
+// 8.5, 6.5, 4100 bytes 33, 27; four, 260 bytes 10.4, 8.3, 4100 bytes 43, 48;
+// sixteen, 132 bytes 18, 14, 260 bytes 15, 22.
+template <int SU, unsigned OWN>
+__device__ __forceinline__ bool better_alone(unsigned mask, unsigned nl, unsigned long long bytes, unsigned mis) {
+  const unsigned mine = bytes < kLong * 16 ? (unsigned)bytes >> 4 : kLong;
+  if (!__any_sync(mask, mine > OWN)) return false;
+  unsigned sms;
+  asm("mov.u32 %0, %%nsmid;" : "=r"(sms));
+  const unsigned warps = gridDim.x * gridDim.y * gridDim.z * ((blockDim.x * blockDim.y * blockDim.z + 31) >> 5);
+  const unsigned most = __reduce_max_sync(mask, (mis & 15) == 0 || ((mis & 3) == 0 && mine <= 32) ? mine : kLong);
+  const unsigned slots = __reduce_add_sync(mask, (mine + nl - 1) / nl);
+  return most < kLong && most * 3 * SU < slots * 32 &&
+         (warps < 2 * sms || (unsigned long long)warps * most < 96ull * sms);
 }
 
 // One copy per calling thread (the thread forms of put and get).  Lanes of a
@@ -572,17 +593,18 @@ __device__ __forceinline__ void copy_own(char *dst, const char *src, unsigned nv
 // is work (see copy_lanes_body).  25,000 calls of log-normal sizes (median
 // 2 KiB, up to 3 MiB, 282 MB moved) took 1240-2060 us with every lane on its
 // own, as long as the longest call takes one thread; together 115-140 us.
-// A lane whose copy has at most kOwn vectors, or operands that are not 4-byte
-// aligned, copies it itself, as do fewer than kTogether lanes, and a lane with
-// an operand in its own local memory, where the same address names another
-// array in every other lane.  LU / SU: the vectors in flight per lane for long
-// and short copies.  FULL: the caller knows that all 32 lanes are here, with
-// operands in the heap.
+// A lane whose copy has at most OWN vectors (one round trip, in parallel with
+// the other lanes), or operands that are not 4-byte aligned, copies it itself,
+// as do fewer than kTogether lanes, and a lane with an operand in its own local
+// memory, where the same address names another array in every other lane.  LU /
+// SU: the vectors in flight per lane for long and short copies.  FULL: the
+// caller knows that all 32 lanes are here, with operands in the heap; without
+// it the lanes also ask better_alone.
 //
 // The first __syncwarp makes what a lane wrote before its call visible to the
 // lanes that copy for it, the last one makes their stores the calling lane's
 // (its later fences and signals order them like its own).
-template <int LU, int SU, bool FULL = false>
+template <int LU, int SU, bool FULL = false, unsigned OWN = 4>
 __device__ __forceinline__ void copy_lanes(char *dst, const char *src, unsigned long long bytes) {
   unsigned mask = 0xffffffffu;
   bool local = false;
@@ -592,7 +614,7 @@ __device__ __forceinline__ void copy_lanes(char *dst, const char *src, unsigned 
   }
   const unsigned nl = FULL ? 32u : __popc(mask);
   const unsigned mis = (unsigned)((uintptr_t)dst ^ (uintptr_t)src);
-  if (!FULL && (local || nl < kTogether)) {
+  if (!FULL && (local || nl < kTogether || better_alone<SU, OWN>(mask, nl, bytes, mis))) {
     // one thread: 16 vector accesses in flight (measured 2.6x the bandwidth of
     // 4 for a 1 MiB put) and an L2 prefetch 64 rounds (16 KiB) ahead: 1 MiB
     // from DRAM 0.90 -> 1.36 GB/s, from L2 1.89 -> 1.81 GB/s
@@ -624,13 +646,13 @@ __device__ __forceinline__ void copy_lanes(char *dst, const char *src, unsigned 
     }
     dst += head;
     src += head;
-    if (nv <= kOwn) {
+    if (nv <= OWN) {
       if ((mis & 15) == 0)
-        copy_own<16>(dst, src, nv);
+        copy_own<16, OWN>(dst, src, nv);
       else if ((mis & 7) == 0)
-        copy_own<8>(dst, src, nv);
+        copy_own<8, OWN>(dst, src, nv);
       else
-        copy_own<4>(dst, src, nv);
+        copy_own<4, OWN>(dst, src, nv);
       nv = 0;
     }
   }
