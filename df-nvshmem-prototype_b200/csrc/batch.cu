@@ -483,28 +483,28 @@ __global__ void __launch_bounds__(256, 3) batch_exec_tma_kernel(const WorkItem *
 }
 
 // ------------------------------------------------ small batches: one launch
-// Below kSmallPerThread requests for each thread of a CTA, planning is done by
-// every CTA for itself: it reads all requests (at most 112 KB, from L2 or, for a
-// few, from the kernel's parameters), checks them, and builds the running count
-// of pieces in its own shared memory.  No CTA waits for another and nothing has
-// to be zeroed, so the memset, the plan kernel and the exec kernel become one
-// launch; an invalid request is seen by every CTA, and none copies anything.
-// Pieces are a power of two of bytes, at most the configured chunk and about two
-// for each warp of the grid, so a batch of few requests still spreads over every
-// SM (with 16 KiB chunks a 64-request batch keeps some 80 of 1184 warps busy).
-// CTA b takes pieces b, b + gridDim.x, ..., its warps the next one each.
+// Small batches (small_limit): planning is done by every CTA for itself.  It
+// reads all requests (at most 128 KB, from L2 or, for a few, from the kernel's
+// parameters), checks them, and builds the running count of pieces in its own
+// shared memory.  No CTA waits for another and nothing has to be zeroed, so the
+// memset, the plan kernel and the exec kernel become one launch; an invalid
+// request is seen by every CTA, and none copies anything.  Pieces are a power of
+// two of bytes, at most the configured chunk and about two for each warp of the
+// grid, so a batch of few requests still spreads over every SM (with 16 KiB
+// chunks a 64-request batch keeps some 80 of 1184 warps busy).  CTA b takes
+// pieces b, b + gridDim.x, ..., its warps the next one each.
 //
-// What it costs is the requests that each thread reads, so that is what limits
-// it.  Times of a call as one launch and as plan and exec (submit from pinned
-// memory; execute), median request 2 KiB:
-//   CTAs of 256 threads, 3 x 8 KiB rings  1000 requests 33, 44; 26, 30 us
-//                                         3000 41, 46; 32, 32   3500 44, 46; 34, 34
-//                                         4095 47, 46; 36, 34
-//   CTAs of 128 threads, 2 x 8 KiB rings  1500 38, 46; 30, 32   2000 40, 46; 33, 33
-//                                         2500 45, 46; 36, 34   4095 53, 48; 42, 35
-// With 2 x 16 KiB rings the lines cross at 1500 and 2200 requests, with rings of
-// 1 to 4 KiB stages at 2500 to 3500.
-constexpr int kSmallPerThread = 14;
+// What it saves is a plan's launches, what it costs the requests that each thread
+// reads: 512 requests, and 12 for each thread of a CTA; 512 more for a submit,
+// which also saves the steps between its copy and the plan.  Times of a call as
+// one launch and planned (median request 2 KiB; submit from pinned memory, us):
+//   CTAs of 256 threads,   submit   3000 requests 41, 46   3600 45, 47   4095 46.5, 46
+//   3 x 8 KiB rings        execute  3000 32, 32   3500 34, 34   4095 36, 34
+//   CTAs of 128 threads,   submit   1800 41, 47   2500 45, 46   3000 48, 48
+//   2 x 8 KiB rings        execute  1500 30, 32   2000 33, 33   2500 36, 34
+// With 2 x 16 KiB rings of 4 warps the lines cross at 2200 (submit) and 1500
+// requests, with rings of 1 to 4 KiB stages at 2500 to 3500, and with 8 warps of
+// 2 x 2 KiB not below 4096.
 constexpr int kParamWords = 240;  // 16-byte words of requests that fit the kernel's parameters
 
 template <int NP>
@@ -1170,11 +1170,14 @@ static SmallParFn pick_small_par(int stages) {
 
 static const size_t kMaxSmem = 227u << 10;
 
+// Below this many requests a batch runs as one launch (see batch_small_kernel).
+static int small_limit(const nvshmemx_batch_config &k, bool submit) { return 512 + 12 * k.threads + (submit ? 512 : 0); }
+
 // Whether n requests run as one launch: a TMA configuration whose rings leave
 // room for the running count (the default's do, up to the limit).
-static bool small_batch(const nvshmemx_batch *b, int n) {
+static bool small_batch(const nvshmemx_batch *b, int n, bool submit) {
   const nvshmemx_batch_config &k = b->cfg;
-  return n > 0 && n < kSmallPerThread * k.threads && k.stream == 0 && k.tma_stages > 0 && small_smem_bytes(k, n) <= kMaxSmem;
+  return n > 0 && n < small_limit(k, submit) && k.stream == 0 && k.tma_stages > 0 && small_smem_bytes(k, n) <= kMaxSmem;
 }
 
 // Enqueues a small batch on the batch's stream: n requests in device memory at
@@ -1259,7 +1262,7 @@ int batch_enqueue_range(nvshmemx_batch *b, int first, int n, const nvshmemx_batc
   int rc;
   // the dispatch of nvshmemx_batch_execute, by which variants are timed: few
   // requests as one launch, whose errors go straight to the sticky word
-  if (small_batch(b, n)) {
+  if (small_batch(b, n, false)) {
     rc = enqueue_small(b, b->d_reqs + first, nullptr, n, false, nullptr, sticky_word(b));
     b->cfg = saved;
     return rc;
@@ -1405,7 +1408,7 @@ int nvshmemx_batch_upload(nvshmemx_batch *b, const nvshmemx_request *reqs, int n
 int nvshmemx_batch_execute(nvshmemx_batch *b, int reps, float *out_ms) {
   if (!b || reps < 1) return fail(NVSHMEMX_ERR_INVALID, "batch_execute: bad arguments");
   int rc;
-  const bool small = small_batch(b, b->n);
+  const bool small = small_batch(b, b->n, false);
   if (!small && (rc = ensure_graph(b, b->d_reqs))) return rc;
   b->last_pieces = 1;
   b->h_status[0] = b->h_status[1] = 0;
@@ -1484,7 +1487,7 @@ int nvshmemx_batch_submit(nvshmemx_batch *b, const nvshmemx_request *reqs, int n
   if (!b || n < 0 || n > b->max_n || (n && !reqs)) return fail(NVSHMEMX_ERR_INVALID, "batch_submit: bad arguments");
   int rc;
   b->n = n;
-  const bool small = small_batch(b, n), two = !b->cfg.stream && n >= kTwoPieces;
+  const bool small = small_batch(b, n, true), two = !b->cfg.stream && n >= kTwoPieces;
   if (!small && !two && (rc = ensure_graph(b, b->d_reqs))) return rc;
   b->last_pieces = 1;
   b->timed_direct = false;
@@ -1531,7 +1534,7 @@ int nvshmemx_batch_submit_compact(nvshmemx_batch *b, const nvshmemx_request_comp
   }
   // the plan kernels expand the compact requests and leave the full form in
   // b->d_reqs
-  const bool small = small_batch(b, n), two = n >= kTwoPieces;
+  const bool small = small_batch(b, n, true), two = n >= kTwoPieces;
   cudaEventRecord(b->ev_start, two ? b->copy_stream : b->stream);
   if ((rc = small ? submit_small(b, reqs, b->d_reqs_compact, sizeof(nvshmemx_request_compact), true, n)
             : two ? submit_two(b, reqs, b->d_reqs_compact, sizeof(nvshmemx_request_compact), kCompact, n)
@@ -1611,7 +1614,7 @@ unsigned long long nvshmemx_requests_bytes(const nvshmemx_request *reqs, int n) 
 }
 
 // Per-call path on the batch's device-resident requests: one caller unit per
-// request through the public device API (nvshmemx_exec_requests' kernel).
+// request (nvshmemx_exec_requests' kernel).
 int nvshmemx_batch_execute_percall(nvshmemx_batch *b, int mode, int reps, float *out_ms) {
   if (!b || reps < 1 || mode < 0 || mode > NVSHMEMX_MODE_BULK)
     return fail(NVSHMEMX_ERR_INVALID, "batch_execute_percall: bad arguments");

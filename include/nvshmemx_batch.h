@@ -6,7 +6,7 @@
  * device API (nvshmem_device.cu:488-540) and the caller decides how many
  * threads issue how many calls.  A batch here is an array of
  * nvshmemx_request descriptors (nvshmemx_ops.h) that one CUDA graph executes
- * with two kernels:
+ * with two kernels (up to some thousand requests, one kernel does both):
  *   plan  -- validates and translates each request and cuts it into chunks of
  *            at most chunk_bytes (a 0-byte SIGNAL/P is one chunk);
  *   exec  -- a persistent grid whose warps claim chunks from a device-wide
@@ -87,9 +87,9 @@ int nvshmemx_batch_execute(nvshmemx_batch *b, int reps, float *out_ms);
 /* End-to-end call: copies n requests from host memory (pinned if it is the
  * batch's host buffer), executes them and reads back the batch status word;
  * *out_status receives the status (0 = every request done), *out_ms the
- * device time of the whole sequence.  Below 14 requests to a
- * thread of a CTA (3584 with the default 256 threads) a TMA configuration runs
- * the batch as one launch (no plan kernel, no graph; the work unit is then at
+ * device time of the whole sequence.  Below 1024 requests
+ * and 12 for each thread of a CTA (4096 with the default 256 threads; 3584 in
+ * nvshmemx_batch_execute) a TMA configuration runs the batch as one launch (no plan kernel, no graph; the work unit is then at
  * most chunk_bytes), and some hundred requests travel as the kernel's
  * parameters.  Otherwise, with a graph configuration (stream 0),
  * the copy precedes the plan and exec kernels on the batch's stream; from
@@ -115,9 +115,10 @@ int nvshmemx_batch_submit(nvshmemx_batch *b, const nvshmemx_request *reqs, int n
 int nvshmemx_batch_submit_compact(nvshmemx_batch *b, const nvshmemx_request_compact *reqs, int n,
                                   int *out_status, float *out_ms);
 
-/* The same work as nvshmemx_batch_execute, enqueued without a graph and with
- * CUDA events around the plan and exec kernels on the batch's stream:
- * *out_ms is the time of all reps, *out_exec_ms the exec kernel's share. */
+/* The batch by its plan and exec kernels, whatever its size (a small one runs
+ * as one launch in nvshmemx_batch_execute), enqueued without a graph and with
+ * CUDA events around both kernels on the batch's stream: *out_ms is the time of
+ * all reps, *out_exec_ms the exec kernel's share. */
 int nvshmemx_batch_execute_direct(nvshmemx_batch *b, int reps, float *out_ms, float *out_exec_ms);
 
 /* Statistics of the last execution: chunk count, and the plan and exec kernel
@@ -130,8 +131,9 @@ int nvshmemx_batch_last_stats(const nvshmemx_batch *b, unsigned long long *chunk
 unsigned long long nvshmemx_requests_bytes(const nvshmemx_request *reqs, int n);
 
 /* The per-call path on the same device-resident requests: one caller unit
- * per request (mode NVSHMEMX_MODE_*) through the public device API, `reps`
- * launches back to back; *out_ms the device time of all reps. */
+ * per request (mode NVSHMEMX_MODE_*) with the checks and results of the public
+ * device calls (puts and gets are copied by the kernel itself), `reps` launches
+ * back to back; *out_ms the device time of all reps. */
 int nvshmemx_batch_execute_percall(nvshmemx_batch *b, int mode, int reps, float *out_ms);
 
 /* Work items (chunks) the allocation-free entry point below can hold:

@@ -1,5 +1,5 @@
 """Batches on both sides of the size up to which one launch plans and executes
-them: 14 requests to a thread of a CTA, for both CTA sizes."""
+them, for both CTA sizes, submitted and executed again."""
 import pytest
 
 from oracle.model import Model
@@ -11,9 +11,10 @@ NPES, HEAP = 4, 32 << 20
 
 
 @pytest.mark.parametrize("threads", [128, 256])
+@pytest.mark.parametrize("base", [512, 1024])
 @pytest.mark.parametrize("extra", [-1, 0])
-def test_one_launch_and_two(shmem_factory, threads, extra):
-    n = 14 * threads + extra
+def test_one_launch_and_two(shmem_factory, threads, base, extra):
+    n = base + 12 * threads + extra
     sh, om = shmem_factory(NPES, HEAP), Model(NPES, HEAP)
     for pe in range(NPES):
         sh.fill_random(pe, 0, HEAP, 22)
