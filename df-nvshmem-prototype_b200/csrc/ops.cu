@@ -1,8 +1,8 @@
-// ops.cu -- host-callable operations (nvshmemx_ops.h) built on the public
-// device API of nvshmem_device.h / nvshmemx.h.  The kernels here are what an
-// application of the prototype writes by hand: they call nvshmem_int_put,
-// nvshmem_int_p, nvshmem_int_wait_until, nvshmem_quiet ... from inside one
-// collective launch in which blockIdx.z is the PE.
+// ops.cu -- host-callable operations (nvshmemx_ops.h): what an application of
+// the prototype writes by hand, in one collective launch in which blockIdx.z is
+// the PE.  The kernels call nvshmem_int_p, nvshmem_int_wait_until, nvshmem_quiet
+// and the barriers of the public device API; their puts and gets have its checks,
+// results and trace records and copy in the kernel itself.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdio.h>

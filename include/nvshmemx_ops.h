@@ -68,14 +68,14 @@ typedef struct nvshmemx_request_compact {
 } nvshmemx_request_compact;
 
 /* How a request is carried out (the per-call variants). */
-#define NVSHMEMX_MODE_THREAD 0 /* one thread per request, nvshmem_{T}_put/get/p/g */
-#define NVSHMEMX_MODE_WARP 1   /* one warp per request, nvshmemx_{T}_put/get_warp  */
-#define NVSHMEMX_MODE_BLOCK 2  /* one CTA per request, nvshmemx_{T}_put/get_block  */
+#define NVSHMEMX_MODE_THREAD 0 /* one thread per request, as nvshmem_{T}_put/get/p/g */
+#define NVSHMEMX_MODE_WARP 1   /* one warp per request, as nvshmemx_{T}_put/get_warp  */
+#define NVSHMEMX_MODE_BLOCK 2  /* one CTA per request, as nvshmemx_{T}_put/get_block  */
 #define NVSHMEMX_MODE_BULK 3   /* one CTA per request, TMA bulk ring               */
 
-/* Runs n requests (host array) as one launch, one caller unit per request,
- * through the public device API; requests must not overlap in their
- * destinations.  *out_ms receives the kernel time (may be NULL). */
+/* Runs n requests (host array) as one launch, one caller unit per request, with
+ * the checks and results of the public device calls (puts and gets are copied by
+ * the kernel itself); requests must not overlap in their destinations.  *out_ms receives the kernel time (may be NULL). */
 int nvshmemx_exec_requests(const nvshmemx_request *reqs, int n, int mode, float *out_ms);
 
 /* ---- deterministic fill and on-device comparison ------------------------- */
@@ -120,8 +120,9 @@ int nvshmemx_op_offload_barrier(int iters, double *out_us_per_call);
  * PE itself is skipped (npes-1 messages per PE).  Each round is followed by
  * nvshmem_quiet and the device barrier.  Round r uses buffer set r % nsets,
  * set s at send_off + s*set_stride / recv_off + s*set_stride, so the working
- * set can exceed L2.  mode: NVSHMEMX_MODE_* (THREAD = one thread per message
- * through nvshmem_{T}_put/get).  dtype selects the typed call for THREAD.
+ * set can exceed L2.  mode: NVSHMEMX_MODE_* (THREAD = one thread per message,
+ * whose warp's lanes copy together).  dtype: the element type, of which `bytes`
+ * is a multiple and which a trace of the THREAD mode names.
  * ctas_per_pe 0: NVSHMEM_CTAS_PER_PE if set, else SMs / npes. */
 int nvshmemx_op_alltoall(int op, int dtype, size_t send_off, size_t recv_off, size_t bytes,
                          int rounds, int nsets, size_t set_stride, int mode, int ctas_per_pe,

@@ -20,9 +20,9 @@ extern "C" {
 
 typedef struct nvshmemx_tune_result {
   nvshmemx_batch_config cfg;
-  float ms_median;  /* median over reps of one graph execution            */
+  float ms_median;  /* median over reps of one nvshmemx_batch_execute      */
   float ms_min;
-  float exec_ms_median;  /* the exec kernel alone (direct path, events)   */
+  float exec_ms_median;  /* the exec kernel alone (plan and exec, events) */
   int status;       /* 0, or the error the candidate hit                    */
 } nvshmemx_tune_result;
 
